@@ -106,6 +106,7 @@ void dev_free(T*& p) {
 void free_lattice(LbmHandle* h) {
     dev_free(h->d_map);
     dev_free(h->d_coord);
+    dev_free(h->d_links);
     dev_free(h->d_tinfo);
     h->d_spt_ctr = nullptr;
     h->spt_base = 0;
@@ -259,6 +260,7 @@ int lbm_set_geometry_strided(LbmHandle* h, const int8_t* solid, int64_t si, int6
     h->have_geometry = h->initialized = h->macros_valid = false;
     int rc = geom_build(h, solid, si, sj, sk);
     if (!rc) rc = sp_tiles_setup(h);
+    if (!rc && !h->f64 && !h->p.two_phase) rc = links_build(h);
     if (rc) { free_lattice(h); return rc; }
     const size_t rbytes = h->f64 ? 8 : 4;
     rc = rc ? rc : dev_alloc(h, &h->d_f[0], h->elem * 19 * h->np, "f_A");
@@ -285,7 +287,9 @@ int lbm_set_geometry_strided(LbmHandle* h, const int8_t* solid, int64_t si, int6
     if (rc) { free_lattice(h); return rc; }
     h->have_geometry = true;
     h->have_psi = false;
-    l2_persist_map(h);
+    // the link steps do not read the map; a window that nothing uses costs the
+    // populations that part of L2 (256^3 pack: 200 us a step with it, 165 without)
+    if (h->f64 || h->p.two_phase || h->tiled) l2_persist_map(h);
     return LBM_OK;
 }
 
@@ -330,6 +334,7 @@ int lbm_set_grey(LbmHandle* h, const double* ns) {
         return rc;
     }
     h->grey = true;
+    if (!h->l2_persist) l2_persist_map(h);   // the grey step reads the map
     return LBM_OK;
 }
 

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/lbm_gb300.h"
+#include "lbm_links.cuh"
 
 #include <nvtx3/nvToolsExt.h>
 
@@ -79,6 +80,8 @@ struct LbmHandle {
     unsigned long long* d_spt_ctr = nullptr;  // its tile claim counter (inside the d_tinfo allocation)
     unsigned long long spt_base = 0;       // counter value at the next launch's first claim
     uint32_t* d_coord = nullptr;           // packed (i,j,k) per node
+    void* d_links = nullptr;               // neighbour links (lbm_links.cuh), one allocation
+    LbmLinks links{};
     void* d_f[2] = {nullptr, nullptr};     // populations, 19 x np elements in AoSoA-32 chunks
     int cur = 0;
     void* d_vprev = nullptr;               // [3][np] previous-step v (pressure faces)
@@ -108,6 +111,8 @@ int lbm_cuda_check(LbmHandle* h, cudaError_t e, const char* what);
 // index construction and dense output (lbm_geom.cu)
 int geom_build(LbmHandle* h, const int8_t* solid, int64_t si, int64_t sj, int64_t sk);
 int geom_host_index(LbmHandle* h);
+// Neighbour links of the index (lbm_links.cu).
+int links_build(LbmHandle* h);
 template <typename O>
 int geom_dense_out(LbmHandle* h, const void* dsrc, int comps, O* out, O fill);
 

@@ -1,0 +1,125 @@
+// Pull gather through the neighbour links (lbm_links.cuh), shared by the step
+// kernels that use them.
+#pragma once
+#include "lbm_common.cuh"
+#include "lbm_internal.h"
+#include "lbm_links.cuh"
+
+namespace lbmk {
+
+// Wait for the previous step (programmatic dependent launch), and hand back the
+// pointer to what it wrote.  The populations must not be read through a const
+// __restrict__ pointer here: such loads count as invariant for the kernel's whole
+// life and may be moved above the wait.
+template <typename T>
+__device__ __forceinline__ const T* wait_previous(const T* p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+
+// A node's links: loaded before the wait (they never change between steps).
+struct NodeLinks {
+    int4 a, b;          // the group's row starts
+    uint32_t w, bits;
+    __device__ __forceinline__ void load(const LbmLinks& L, int n) {
+        const int4* head = reinterpret_cast<const int4*>(L.head + n / LBM_LINK_GROUP);
+        a = __ldg(head);
+        b = __ldg(head + 1);
+        const uint2 x = __ldg(L.node + n);
+        w = x.x;
+        bits = x.y;
+    }
+    // Node across in row r.
+    template <int RW>
+    __device__ __forceinline__ int rank() const {
+        const int4& h = RW < 4 ? a : b;
+        const int start = (RW & 3) == 0 ? h.x : (RW & 3) == 1 ? h.y : (RW & 3) == 2 ? h.z : h.w;
+        const uint32_t q = RW < 6 ? w >> (5 * RW) & 31u : bits >> (22 + 5 * (RW - 6)) & 31u;
+        return start + (int)(threadIdx.x & 31) + (int)q;
+    }
+};
+
+// Reference density of the 16-bit codecs at a node and its sources at x - 1 and
+// x + 1: stepped from the node's own value in a warp without an x face, from
+// the wrapped x in the others (the rounding of gather_node).
+template <typename R>
+struct LinkRef {
+    R at, xm, xp;
+    __device__ __forceinline__ LinkRef(const LbmRef<R>& ref, int i, int nx) {
+        const bool inside = __all_sync(__activemask(), i > 0 && i < nx - 1);
+        at = lbm_ref_at(ref, i);
+        xm = inside ? at - ref.b : lbm_fma<R>(ref.b, (R)(i == 0 ? nx - 1 : i - 1), ref.a);
+        xp = inside ? at + ref.b : lbm_fma<R>(ref.b, (R)(i == nx - 1 ? 0 : i + 1), ref.a);
+    }
+    template <int S>
+    __device__ __forceinline__ R of() const {
+        return lbm_ex(S) > 0 ? xm : (lbm_ex(S) < 0 ? xp : at);
+    }
+};
+
+// All of a node's pulled populations.  Direction s and its opposite are
+// neighbours in the slot order, so the own opposite slot is the own slot s moved
+// by one: both candidates of the load share the immediate offset of slot s.
+template <int STORE, bool REF>
+struct LinkGather {
+    using Cd = Codec<STORE>;
+    using T = typename Cd::T;
+    using R = typename Cd::R;
+    template <int S>
+    static __device__ __forceinline__ void one(R* F, const T* fin, int own, int src, uint32_t bits, const LinkRef<R>& rx) {
+        const bool bounce = bits >> S & 1u;
+        const int a = bounce ? own + 32 * (lbm_lr(S) - S) : lbm_eoff32(src);
+        F[S] = Cd::template dec<S>(fin[a + 32 * S]);
+        if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), bounce ? rx.at : rx.template of<S>(), F[S]);
+    }
+    template <int RW>
+    static __device__ __forceinline__ void row(R* F, const T* fin, int own, const NodeLinks& K, const LinkRef<R>& rx) {
+        constexpr int c = lbm_link_dir(RW, 0);
+        const int m = K.template rank<RW>();
+        one<c>(F, fin, own, m, K.bits, rx);
+        if constexpr (RW < 4) {
+            one<lbm_link_dir(RW, 1)>(F, fin, own, m - 1, K.bits, rx);
+            // x + 1 ranks after x only where x itself is fluid
+            one<lbm_link_dir(RW, -1)>(F, fin, own, m + (int)(~K.bits >> c & 1u), K.bits, rx);
+        }
+    }
+    // Explicit sources of the links that the node word cannot express; a warp
+    // holds one group.
+    static __device__ __forceinline__ void recorded(R* F, const T* fin, const LbmLinks& L, int n, uint32_t bits,
+                                                    const LinkRef<R>& rx) {
+        const uint32_t e = __ballot_sync(__activemask(), bits & LBM_LINK_EXC);
+        if (!(bits & LBM_LINK_EXC)) return;
+        const int first = __ldg(L.rec0 + n / LBM_LINK_GROUP);
+        const int32_t* rec = L.rec + (int64_t)LBM_LINK_REC * (first + __popc(e & ((1u << (threadIdx.x & 31)) - 1u)));
+#define LBM_X(S)                                                                              \
+    {                                                                                         \
+        const int src = __ldg(rec + S);                                                       \
+        if (src >= 0) {                                                                       \
+            F[S] = Cd::template dec<S>(fin[lbm_eoff32(src) + 32 * S]);                        \
+            if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), rx.template of<S>(), F[S]);     \
+        }                                                                                     \
+    }
+        LBM_ALL_DIRS(LBM_X)
+#undef LBM_X
+    }
+    static __device__ __forceinline__ void all(R* F, const T* fin, const LbmLinks& L, const NodeLinks& K, int n,
+                                               const LinkRef<R>& rx) {
+        const int own = lbm_eoff32(n);
+        F[0] = Cd::template dec<0>(fin[own]);
+        if constexpr (REF) F[0] = lbm_fma<R>((R)lbm_w(0), rx.at, F[0]);
+        one<1>(F, fin, own, n - 1, K.bits, rx);
+        one<2>(F, fin, own, n + 1, K.bits, rx);
+        row<0>(F, fin, own, K, rx);
+        row<1>(F, fin, own, K, rx);
+        row<2>(F, fin, own, K, rx);
+        row<3>(F, fin, own, K, rx);
+        row<4>(F, fin, own, K, rx);
+        row<5>(F, fin, own, K, rx);
+        row<6>(F, fin, own, K, rx);
+        row<7>(F, fin, own, K, rx);
+        recorded(F, fin, L, n, K.bits, rx);
+    }
+};
+
+}  // namespace lbmk

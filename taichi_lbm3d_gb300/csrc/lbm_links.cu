@@ -1,0 +1,196 @@
+// Builds the neighbour links (lbm_links.cuh) of a lattice from its dense map
+// and packed coordinates: one warp per group of 32 nodes, two passes (tables
+// and record counts, then the records).
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "lbm_common.cuh"
+#include "lbm_internal.h"
+#include "lbm_links.cuh"
+
+namespace {
+
+struct LinkBuild {
+    const int32_t* map;
+    const uint32_t* coord;
+    int32_t nx, ny, nz, n_fluid;
+    int32_t bc[6];
+    int32_t bc_form;
+    uint2* node;
+    LbmLinkHead* head;
+    int32_t* rec0;
+    int32_t* rec;
+    int32_t cap;          // records allocated
+    int32_t* total;       // records needed
+};
+
+struct Row {
+    int src[3];           // sources at x - 1, x, x + 1 (wrapped), -1 solid
+    bool cross[3];        // the link crosses a periodic face
+    int rank;             // rank of the cell across, -1 when no link of the row needs it
+};
+
+// Links of the row (e_y, e_z) of a node; WIDE: the row's three cells, else the one across.
+template <bool WIDE>
+__device__ __forceinline__ Row link_row(const LinkBuild& B, int ey, int ez, int i, int j, int k) {
+    const int y = j - ey, z = k - ez;
+    const int yw = y < 0 ? B.ny - 1 : (y >= B.ny ? 0 : y), zw = z < 0 ? B.nz - 1 : (z >= B.nz ? 0 : z);
+    const int64_t row = (int64_t)B.nx * (yw + (int64_t)B.ny * zw);
+    Row o;
+    o.rank = -1;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        o.src[d] = -1;
+        o.cross[d] = false;
+        if (!WIDE && d != 1) continue;
+        const int x = i + d - 1;
+        const int xw = x < 0 ? B.nx - 1 : (x >= B.nx ? 0 : x);
+        o.cross[d] = x != xw || y != yw || z != zw;
+        o.src[d] = __ldg(B.map + row + xw);
+    }
+    if (o.src[1] >= 0 && !o.cross[1]) o.rank = o.src[1];
+    else if (o.src[0] >= 0 && !o.cross[0]) o.rank = o.src[0] + 1;
+    else if (o.src[2] >= 0 && !o.cross[2]) o.rank = o.src[2];
+    return o;
+}
+
+template <bool FILL>
+__global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int ngroup) {
+    const int group = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (group >= ngroup) return;
+    const int n = group * LBM_LINK_GROUP + lane;
+    const bool live = n < B.n_fluid;
+    const uint32_t pc = live ? B.coord[n] : 0u;
+    const int i = lbm_pi(pc), j = lbm_pj(pc), k = lbm_pk(pc);
+    uint32_t bits = live ? 0u : 0x7fffeu;   // padding: every direction from the own slots
+    bool whole = false;                     // a face condition replaces all that the node pulls
+    Row own{};
+    if (live) {
+        const bool at[6] = {i == 0, i == B.nx - 1, j == 0, j == B.ny - 1, k == 0, k == B.nz - 1};
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            if (!at[f] || B.bc[f] == LBM_BC_PERIODIC) continue;
+            bits |= LBM_LINK_FACE;
+            if (B.bc[f] == LBM_BC_PRESSURE) bits |= LBM_LINK_PRESSURE;
+            // (the in-place velocity form reads what was pulled)
+            whole |= B.bc[f] == LBM_BC_PRESSURE || B.bc_form == 0;
+        }
+        own = link_row<true>(B, 0, 0, i, j, k);
+#pragma unroll
+        for (int d = 0; d < 3; d += 2) {
+            if (own.src[d] < 0 || own.cross[d]) bits |= d ? 4u : 2u;
+            if (own.src[d] >= 0 && own.cross[d] && !whole) bits |= LBM_LINK_EXC;
+        }
+    }
+    int start[8];
+    uint32_t w0 = 0, w1 = 0, far = 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        int rank = -1;
+        if (live) {
+            const Row o = r < 4 ? link_row<true>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k)
+                                : link_row<false>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k);
+            rank = o.rank;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                if (r >= 4 && d != 1) continue;
+                const int s = lbm_link_dir(r, 1 - d);   // source x + d - 1 belongs to e_x = 1 - d
+                if (o.src[d] < 0 || o.cross[d]) bits |= 1u << s;
+                if (o.src[d] >= 0 && o.cross[d] && !whole) bits |= LBM_LINK_EXC;
+            }
+        }
+        start[r] = __reduce_min_sync(0xffffffffu, rank >= 0 ? rank - lane : 0x7fffffff);
+        if (start[r] == 0x7fffffff) start[r] = 0;
+        uint32_t q = rank >= 0 ? (uint32_t)(rank - lane - start[r]) : 0u;
+        if (q > 31u) {
+            q = 0;
+            far |= 1u << r;
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (r < 4 || d == 1) bits |= 1u << lbm_link_dir(r, 1 - d);
+            if (!whole) bits |= LBM_LINK_EXC;
+        }
+        if (r < 6) w0 |= q << (5 * r);
+        else w1 |= q << (22 + 5 * (r - 6));
+    }
+    const uint32_t exc = __ballot_sync(0xffffffffu, bits & LBM_LINK_EXC);
+    if constexpr (!FILL) {
+        int v = start[0];
+#pragma unroll
+        for (int r = 1; r < 8; ++r)
+            if (lane == r) v = start[r];
+        if (lane < 8) B.head[group].start[lane] = v;
+        if (lane == 0) B.rec0[group] = exc ? atomicAdd(B.total, __popc(exc)) : 0;
+        B.node[n] = make_uint2(w0, w1 | bits);
+    } else if (bits & LBM_LINK_EXC) {
+        const int slot = B.rec0[group] + __popc(exc & ((1u << lane) - 1u));
+        if (slot >= B.cap) return;               // the host allocates more and builds again
+        int32_t* out = B.rec + (int64_t)LBM_LINK_REC * slot;
+        out[0] = out[19] = -1;
+        out[1] = own.cross[0] ? own.src[0] : -1;
+        out[2] = own.cross[2] ? own.src[2] : -1;
+#pragma unroll 1
+        for (int r = 0; r < 8; ++r) {
+            const Row o = link_row<true>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k);
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                if (r < 4 || d == 1) out[lbm_link_dir(r, 1 - d)] = o.cross[d] || (far >> r & 1u) ? o.src[d] : -1;
+        }
+    }
+}
+
+}  // namespace
+
+// Links of the lattice whose map and coordinates are on the device; one
+// allocation (h->d_links).  Records: room for every node of the periodic faces;
+// a geometry that needs more (rows far from a line) gets a second one.
+int links_build(LbmHandle* h) {
+    const LbmParams& p = h->p;
+    const int64_t ngroup = h->np / LBM_LINK_GROUP;
+    int64_t cap = 0;
+    const int64_t area[3] = {(int64_t)p.ny * p.nz, (int64_t)p.nx * p.nz, (int64_t)p.nx * p.ny};
+    for (int f = 0; f < 6; ++f)
+        if (p.bc[f] == LBM_BC_PERIODIC || (p.bc[f] == LBM_BC_VELOCITY && p.bc_form != 0)) cap += area[f / 2];
+    cap = std::min<int64_t>(cap, h->n_fluid) + h->n_fluid / 512 + 32;
+    for (;;) {
+        const size_t node = sizeof(uint2) * h->np, head = sizeof(LbmLinkHead) * ngroup;
+        const size_t rec0 = (sizeof(int32_t) * (ngroup + 1) + 15) / 16 * 16;   // + the count
+        const size_t bytes = node + head + rec0 + sizeof(int32_t) * LBM_LINK_REC * cap;
+        int rc = lbm_cuda_check(h, cudaMalloc(&h->d_links, bytes), "neighbour links");
+        if (rc) {
+            h->d_links = nullptr;
+            return rc;
+        }
+        h->device_bytes += (int64_t)bytes;
+        char* at = (char*)h->d_links;
+        LinkBuild B{};
+        B.map = h->d_map;
+        B.coord = h->d_coord;
+        B.nx = p.nx; B.ny = p.ny; B.nz = p.nz;
+        B.n_fluid = h->n_fluid;
+        for (int f = 0; f < 6; ++f) B.bc[f] = p.bc[f];
+        B.bc_form = p.bc_form;
+        B.node = (uint2*)at;
+        B.head = (LbmLinkHead*)(at + node);
+        B.rec0 = (int32_t*)(at + node + head);
+        B.total = B.rec0 + ngroup;
+        B.rec = (int32_t*)(at + node + head + rec0);
+        B.cap = (int32_t)cap;
+        h->links = {B.node, B.head, B.rec0, B.rec};
+        rc = lbm_cuda_check(h, cudaMemsetAsync(B.total, 0, sizeof(int32_t), h->stream), "link records");
+        if (rc) return rc;
+        const int grid = (int)((ngroup + 3) / 4);
+        link_build_kernel<false><<<grid, 128, 0, h->stream>>>(B, (int)ngroup);
+        link_build_kernel<true><<<grid, 128, 0, h->stream>>>(B, (int)ngroup);
+        rc = lbm_cuda_check(h, cudaGetLastError(), "link_build_kernel launch");
+        int32_t total = 0;
+        if (!rc) rc = lbm_cuda_check(h, cudaMemcpyAsync(&total, B.total, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream), "link records");
+        if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "neighbour links");
+        if (rc || total <= cap) return rc;
+        cudaFree(h->d_links);
+        h->d_links = nullptr;
+        h->device_bytes -= (int64_t)bytes;
+        cap = total;
+    }
+}

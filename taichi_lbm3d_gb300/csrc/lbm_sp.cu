@@ -33,6 +33,7 @@
 #include "lbm_common.cuh"
 #include "lbm_internal.h"
 #include "lbm_kernels.cuh"
+#include "lbm_linkgather.cuh"
 
 // Resident 256-thread CTAs per SM requested for the step kernel (caps
 // registers at 65536 / (256 * n)), as measured on the 256^3 pack (MLUPS):
@@ -65,24 +66,18 @@
 namespace {
 using namespace lbmk;
 
-// Everything after the gather: faces, macros, collision and store of node n.
+// Macros, collision and store of node n (faces done); ref: its reference density.
 template <int STORE, bool FORCE, bool MACROS>
-__device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int n, int i, int j, int k,
-                                               const SpConsts<typename Codec<STORE>::R>& C,
-                                               typename Codec<STORE>::T* __restrict__ fout,
-                                               const int32_t* __restrict__ map,
-                                               typename Codec<STORE>::R* __restrict__ vprev,
-                                               typename Codec<STORE>::R* __restrict__ rho_out,
-                                               typename Codec<STORE>::R* __restrict__ v_out) {
+__device__ __forceinline__ void sp_collide_node(typename Codec<STORE>::R* F, int n, bool pressure_face,
+                                                typename Codec<STORE>::R ref,
+                                                const SpConsts<typename Codec<STORE>::R>& C,
+                                                typename Codec<STORE>::T* __restrict__ fout,
+                                                typename Codec<STORE>::R* __restrict__ vprev,
+                                                typename Codec<STORE>::R* __restrict__ rho_out,
+                                                typename Codec<STORE>::R* __restrict__ v_out) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
     const int64_t np = C.np;
-    // Face nodes are rare; warps without one skip the branch uniformly.
-    bool face = false;
-    if (C.any_bc) {
-        face = on_face(i, j, k, C, false);
-        if (face) apply_faces<R, Cd::DEV>(F, i, j, k, n, C, map, vprev);
-    }
 
     // macros (SP:376-388); in deviation form r = rho - 1 and rho = 1 + r
     R r = F[0];
@@ -98,7 +93,7 @@ __device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int 
         vy = vy + C.fhalf[1] / rho;
         vz = vz + C.fhalf[2] / rho;
     }
-    if (face && C.any_pressure && on_face(i, j, k, C, true)) {
+    if (pressure_face) {
         vprev[n] = vx;
         vprev[np + n] = vy;
         vprev[2 * np + n] = vz;
@@ -111,7 +106,27 @@ __device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int 
     }
 
     collide_sp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, C);
-    store_node<STORE>(F, fout, n, lbm_ref_at(sp_ref(C), i), C.seed);
+    store_node<STORE>(F, fout, n, ref, C.seed);
+}
+
+// Everything after the gather: faces, macros, collision and store of node n.
+template <int STORE, bool FORCE, bool MACROS>
+__device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int n, int i, int j, int k,
+                                               const SpConsts<typename Codec<STORE>::R>& C,
+                                               typename Codec<STORE>::T* __restrict__ fout,
+                                               const int32_t* __restrict__ map,
+                                               typename Codec<STORE>::R* __restrict__ vprev,
+                                               typename Codec<STORE>::R* __restrict__ rho_out,
+                                               typename Codec<STORE>::R* __restrict__ v_out) {
+    using Cd = Codec<STORE>;
+    // Face nodes are rare; warps without one skip the branch uniformly.
+    bool face = false;
+    if (C.any_bc) {
+        face = on_face(i, j, k, C, false);
+        if (face) apply_faces<typename Cd::R, Cd::DEV>(F, i, j, k, n, C, map, vprev);
+    }
+    sp_collide_node<STORE, FORCE, MACROS>(F, n, face && C.any_pressure && on_face(i, j, k, C, true),
+                                          lbm_ref_at(sp_ref(C), i), C, fout, vprev, rho_out, v_out);
 }
 
 template <int STORE, bool FORCE, bool MACROS>
@@ -153,6 +168,59 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1
     R F[19];
     gather_node<STORE>(F, fin, map, n, C.nx, C.ny, C.nz, i, j, k, sp_ref(C));
     sp_finish_node<STORE, FORCE, MACROS>(F, n, i, j, k, C, fout, map, vprev, rho_out, v_out);
+}
+
+// ------------------------------------------------------------ link step
+// The step of all storages but FP64: the pull sources come from the neighbour
+// links (lbm_links.cuh, 9 bytes a node read in order) instead of coordinates and
+// 18 map lookups.  What that buys is instructions (877 against 1052 per warp of
+// 32 nodes, FP32; 717 against 890, FP32 deviation form) and one dependent load
+// less before the populations.  On the 256^3 pack, MLUPS, map kernel / link kernel:
+// FP32 33.6k / 35.5k, FP32 deviation form 35.1k / 36.1k, FP16 32.2k / 39.9k;
+// 64^3 cavity FP32 30.1k / 34.3k; forced FP32 channel 101 x 67 x 53 19.3k / 21.3k.
+// FP32 then moves 166 B a node at 0.91 of the copy bandwidth (DRAM-bound); the
+// 16-bit storages and the forced FP32 kernel are bound by issue slots.  Two
+// nodes per thread in packed FP32 halve the instructions and were slower (28.0k
+// FP32, 96 registers: half the warps, each living longer), pushing instead of
+// pulling too (19.5k: unaligned stores leave partly written sectors).
+//
+// Resident 128-thread CTAs per SM, measured on the same lattices: 10 (48
+// registers, no spill; FP32 35.5k against 34.4k at 9 and 34.9k at 12, FP16 39.9k
+// against 38.8k at 9 and 39.7k at 11), forced FP32 9 (21.3k against 20.7k at 8).
+#ifndef LBM_LINK_MINBLOCKS
+#define LBM_LINK_MINBLOCKS 10
+#endif
+#ifndef LBM_LINK_MINBLOCKS_F
+#define LBM_LINK_MINBLOCKS_F 9
+#endif
+constexpr int LINK_THREADS = 128;
+
+// REF: 16-bit storage against a reference density that is not 0 everywhere.
+template <int STORE, bool FORCE, bool MACROS, bool REF>
+__global__ void __launch_bounds__(LINK_THREADS, FORCE && !Codec<STORE>::DEV ? LBM_LINK_MINBLOCKS_F : LBM_LINK_MINBLOCKS)
+    sp_link_kernel(const __grid_constant__ SpConsts<float> C, const typename Codec<STORE>::T* f_prev,
+                   typename Codec<STORE>::T* __restrict__ fout, const __grid_constant__ LbmLinks L,
+                   const int32_t* __restrict__ map, const uint32_t* __restrict__ coord, float* __restrict__ vprev,
+                   float* __restrict__ rho_out, float* __restrict__ v_out) {
+    using Cd = Codec<STORE>;
+#if LBM_SP_PDL
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+#endif
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= C.n_fluid) return;
+    NodeLinks K;
+    K.load(L, n);
+    int i = 0;
+    if constexpr (REF) i = lbm_pi(__ldg(coord + n));
+    const LinkRef<float> rx(sp_ref(C), i, C.nx);
+    const auto* fin = wait_previous(f_prev);
+    float F[19];
+    LinkGather<STORE, REF>::all(F, fin, L, K, n, rx);
+    if (K.bits & LBM_LINK_FACE) {
+        const uint32_t pc = __ldg(coord + n);
+        apply_faces<float, Cd::DEV>(F, lbm_pi(pc), lbm_pj(pc), lbm_pk(pc), n, C, map, vprev);
+    }
+    sp_collide_node<STORE, FORCE, MACROS>(F, n, K.bits & LBM_LINK_PRESSURE, rx.at, C, fout, vprev, rho_out, v_out);
 }
 
 // ------------------------------------------------------------ staged step
@@ -621,6 +689,52 @@ int run_tiles(LbmHandle* h, int32_t n, bool macros_last) {
     return LBM_OK;
 }
 
+template <int STORE, bool FORCE, bool MACROS, bool REF>
+int launch_link(LbmHandle* h, const SpConsts<float>& C) {
+    using T = typename Codec<STORE>::T;
+    const T* fin = (const T*)h->d_f[h->cur];
+    T* fout = (T*)h->d_f[h->cur ^ 1];
+    cudaLaunchConfig_t cfg = {};
+    const int block = std::min<int>(h->block, LINK_THREADS);
+    cfg.gridDim = dim3((unsigned)((h->n_fluid + block - 1) / block));
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = h->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = LBM_SP_PDL ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, sp_link_kernel<STORE, FORCE, MACROS, REF>, C, fin, fout, h->links,
+                                             (const int32_t*)h->d_map, (const uint32_t*)h->d_coord, (float*)h->d_vprev,
+                                             (float*)h->d_rho, (float*)h->d_v);
+    h->cur ^= 1;
+    return lbm_cuda_check(h, e != cudaSuccess ? e : cudaGetLastError(), "sp_link_kernel launch");
+}
+
+template <int STORE, bool FORCE, bool REF>
+int run_links_t(LbmHandle* h, int32_t n, bool macros_last) {
+    SpConsts<float> C = sp_make_consts<float>(h);
+    for (int32_t it = 0; it < n; ++it) {
+        C.seed = (uint32_t)(h->steps_done + it);   // global step index: rounding bits of this step
+        const int rc = macros_last && it == n - 1 ? launch_link<STORE, FORCE, true, REF>(h, C)
+                                                  : launch_link<STORE, FORCE, false, REF>(h, C);
+        if (rc) return rc;
+    }
+    return LBM_OK;
+}
+
+template <int STORE>
+int run_links(LbmHandle* h, int32_t n, bool macros_last) {
+    if constexpr (Codec<STORE>::RHOREF) {
+        const SpConsts<float> C = sp_make_consts<float>(h);
+        if (C.ref_a != 0.0f || C.ref_b != 0.0f)
+            return h->force ? run_links_t<STORE, true, true>(h, n, macros_last)
+                            : run_links_t<STORE, false, true>(h, n, macros_last);
+    }
+    return h->force ? run_links_t<STORE, true, false>(h, n, macros_last)
+                    : run_links_t<STORE, false, false>(h, n, macros_last);
+}
+
 template <int STORE>
 int run_steps(LbmHandle* h, int32_t n, bool macros_last) {
     using R = typename Codec<STORE>::R;
@@ -633,6 +747,10 @@ int run_steps(LbmHandle* h, int32_t n, bool macros_last) {
     if (rc0) return rc0;
 #endif
     if (h->tiled) return run_tiles<STORE>(h, n, macros_last);
+#ifndef LBM_DEBUG
+    // (debug builds keep the kernel whose map lookups they check)
+    if constexpr (STORE != LBM_STORE_F64) return run_links<STORE>(h, n, macros_last);
+#endif
     const int grid = (int)((h->n_fluid + h->block - 1) / h->block);
     for (int32_t it = 0; it < n; ++it) {
         const bool mac = macros_last && it == n - 1;

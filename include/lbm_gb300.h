@@ -196,14 +196,14 @@ int lbm_debug_stream(LbmHandle* h, const float* f_in, float* f_out);
 /* ------------------------------------------------------------------ batches
  * Many independent porous subvolumes (no counterpart in the reference, which
  * runs one lattice per process): all faces periodic, shared parameters, one
- * persistent kernel per time step over all active subvolumes, check_every
+ * kernel per time step over all active subvolumes, check_every
  * steps captured in one CUDA graph.  dims: [n_sub][3]; solids: the n_sub
  * x-fastest masks back to back. */
 typedef struct LbmBatch LbmBatch;
 int lbm_batch_create(const LbmParams* params, int32_t n_sub, const int32_t* dims, const int8_t* solids,
                      LbmBatch** out);
 int lbm_batch_destroy(LbmBatch* b);
-/* Work-tile length in nodes per subvolume and CTA size of the persistent kernel
+/* Tile length in nodes per subvolume (at most the CTA's threads) and CTA size of the kernel
  * (chosen by the autotuner in taichi_lbm3d_gb300/autotune.py). */
 int lbm_batch_configure(LbmBatch* b, const int32_t* tile_len, int32_t block);
 /* Rest state f = feq(1, 0) in every subvolume, all subvolumes active. */

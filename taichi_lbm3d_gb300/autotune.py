@@ -1,6 +1,6 @@
-"""Autotuner for the batched persistent kernel.
+"""Autotuner for the batched step kernel.
 
-For each subvolume edge size it times the persistent step kernel over a small
+For each subvolume edge size it times the step kernel over a small
 batch of subvolumes of that size for every candidate (work-tile length, CTA
 size), with CUDA events on the batch's stream, and keeps the fastest.  Results
 are cached in a JSON file keyed by GPU name, storage mode and edge size
@@ -47,7 +47,7 @@ def _gpu_name():
 
 
 def time_config(batch, tile, block, steps=20, warmup=4):
-    """Seconds per step of the persistent kernel with (tile, block)."""
+    """Seconds per step of the kernel with (tile, block)."""
     import torch
     batch.configure([tile] * batch.n, block)
     batch.init()

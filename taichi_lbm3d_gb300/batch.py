@@ -1,8 +1,8 @@
 """Batched permeability of many independent porous subvolumes on one GPU.
 
-One persistent kernel per time step advances every active subvolume (work
-tiles claimed from an atomic counter), ``check_every`` steps are captured into
-one CUDA graph, converged subvolumes leave the work list (csrc/lbm_batch.cu).
+One launch per time step advances every active subvolume (a CTA per tile of its
+nodes), ``check_every`` steps are captured into one CUDA graph, converged
+subvolumes leave the tile list (csrc/lbm_batch.cu).
 Tile lengths and the CTA size come from the project's autotuner
 (``autotune.py``), cached in a JSON file.
 

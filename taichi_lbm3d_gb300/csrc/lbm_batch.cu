@@ -1,19 +1,17 @@
-// K5: many independent porous subvolumes advanced by one persistent kernel per
-// time step, `check_every` steps captured into one CUDA graph.
+// K5: many independent porous subvolumes advanced together, one launch per time
+// step, `check_every` steps captured into one CUDA graph.
 //
 // Layout: the compacted fluid nodes of all subvolumes are concatenated (each
 // subvolume starts on a multiple of 32 so no population chunk straddles two);
-// each subvolume has its own dense node map holding node indices local to the
-// subvolume.  A CTA offsets the population, coordinate and density-reference
-// arrays to its subvolume's first node once (64-bit), and the 32-bit offset
+// each subvolume has its own dense node map and neighbour links holding node
+// indices local to the subvolume.  A CTA offsets the population and link arrays
+// to its subvolume's first node once (64-bit), and the 32-bit offset
 // arithmetic of the gather stays local, so the batch as a whole may exceed
 // 2^31 population elements.  Work is cut into tiles (subvolume, local node
-// range); the grid is sized to the resident CTAs of
-// the GPU and CTAs claim tiles from an atomic counter, so uneven subvolumes
-// share the GPU without tail effects.  Converged subvolumes are removed by
-// rewriting the tile list in device memory between graph launches; the graph
-// itself never changes.  The node update is the single-phase step of K1 (all
-// faces periodic, optional body force) in any storage mode.
+// range), one CTA each, one thread a node.  Converged subvolumes leave the tile list, which is
+// rewritten in device memory and the graph captured again.  The node update is
+// the single-phase step of K1 (all faces periodic, optional body force) in any
+// storage mode.
 //
 // Convergence: the last step of each graph writes, per tile, the FP64 sum of
 // v along x; the host sums tiles in order per subvolume (deterministic) and
@@ -26,15 +24,14 @@
 #include <vector>
 
 #include "lbm_kernels.cuh"
+#include "lbm_linkgather.cuh"
 
-struct BatchSub {
-    int32_t nx, ny, nz, n_fluid;
-    int64_t map_off;        // first cell of this subvolume's dense map
-    int64_t node_begin;     // first node (a multiple of 32) in the concatenated arrays
-};
+using BatchSub = LbmLinkLattice;
 
 struct BatchTile {
-    int32_t sub, begin, end, pad;   // local node range [begin, end)
+    int32_t first32;        // first node of the subvolume / 32
+    int32_t begin, end;     // local node range (begin a multiple of 32)
+    int32_t sub;
 };
 
 // Per-subvolume views of the concatenated arrays (node indices become local).
@@ -55,84 +52,76 @@ struct LbmBatch {
     std::vector<BatchTile> tiles;       // current (active) tile list
     BatchSub* d_subs = nullptr;
     BatchTile* d_tiles = nullptr;
-    int32_t* d_ntiles = nullptr;
-    int32_t* d_counters = nullptr;      // one per step of a graph
+    uint32_t* d_seed = nullptr;         // first step of the launch group (16-bit rounding seed)
     double* d_partial = nullptr;        // per tile
     int64_t max_tiles = 0;
-    int32_t grid = 0, block = 256;
+    int32_t block = 128;
     cudaGraphExec_t graph = nullptr;
     int32_t graph_steps = 0;
     std::vector<int64_t> steps;         // per subvolume
     uint32_t seed_step = 0;             // steps taken since init (16-bit rounding seed)
 };
 
-static const uint32_t* seed_base(const LbmBatch* b) { return reinterpret_cast<const uint32_t*>(b->d_counters + 4096); }
-
 namespace {
 using namespace lbmk;
 
+// One CTA per tile, steps in programmatic dependent launch: tile and links are
+// loaded while the step before drains.  Eight subvolumes of edges 48 to 160 (4.07 M
+// fluid nodes, body force), MLUPS, against a persistent grid whose CTAs claimed
+// 1024-node tiles from a counter and looked sources up in the dense maps: FP16
+// 38.0k / 32.0k, FP32 deviation form 36.3k / 30.9k, FP32 23.5k / 20.2k.  Bound by
+// issue slots as the single-lattice kernel.  Tiles of 64 and 128 threads run
+// alike (38.1k, 38.0k FP16), of 256 36.0k.
 template <int STORE, bool FORCE, bool CHECK>
-__global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : 4) batch_step_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C,
-                                                         const BatchSub* __restrict__ subs,
-                                                         const BatchTile* __restrict__ tiles,
-                                                         const int32_t* __restrict__ n_tiles, int32_t* counter,
-                                                         const typename Codec<STORE>::T* __restrict__ fin,
-                                                         typename Codec<STORE>::T* __restrict__ fout,
-                                                         const int32_t* __restrict__ map,
-                                                         const uint32_t* __restrict__ coord,
-                                                         const uint32_t* __restrict__ seed_base,
-                                                         double* __restrict__ partial) {
+__global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Codec<STORE>::DEV ? 4 : 5)
+    batch_step_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C, const BatchTile* __restrict__ tiles,
+                      const typename Codec<STORE>::T* f_prev, typename Codec<STORE>::T* __restrict__ fout,
+                      const __grid_constant__ LbmLinks links, const uint32_t* __restrict__ seed_base,
+                      double* __restrict__ partial) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
-    __shared__ int s_tile;
     __shared__ double s_red[32];
-    const int nt = *n_tiles;
-    for (;;) {
-        if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1);
-        __syncthreads();
-        const int t = s_tile;
-        __syncthreads();
-        if (t >= nt) return;
-        const BatchTile tl = tiles[t];
-        const BatchSub sd = subs[tl.sub];
-        const int32_t* smap = map + sd.map_off;
-        const typename Cd::T* sfin = sub_pop(fin, sd.node_begin);
-        typename Cd::T* sfout = sub_pop(fout, sd.node_begin);
-        const uint32_t* scoord = coord + sd.node_begin;
-        // 16-bit codecs: all faces periodic, so the reference density is 0; the
-        // rounding bits are those of a single lattice at the same step (step
-        // index = the launch group's first step, set before the group, + k)
-        const uint32_t seed = *seed_base + C.seed;
-        double acc = 0.0;
-        for (int n = tl.begin + threadIdx.x; n < tl.end; n += blockDim.x) {
-            const uint32_t pc = __ldg(scoord + n);
-            const int i = lbm_pi(pc), j = lbm_pj(pc), k = lbm_pk(pc);
-            R F[19];
-            gather_node<STORE>(F, sfin, smap, n, sd.nx, sd.ny, sd.nz, i, j, k);
-            R r = F[0];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int4 t4 = __ldg(reinterpret_cast<const int4*>(tiles + blockIdx.x));
+    const int64_t first = (int64_t)t4.x * 32;
+    const LbmLinks L{links.node + first, links.head + t4.x, links.rec0 + t4.x, links.rec};
+    const int n = t4.y + threadIdx.x;
+    const bool live = n < t4.z;
+    NodeLinks K;
+    K.load(L, live ? n : t4.y);
+    // 16-bit codecs: all faces periodic, so the reference density is 0; the
+    // rounding bits are those of a single lattice at the same step (step
+    // index = the launch group's first step, set before the group, + k)
+    const uint32_t seed = *seed_base + C.seed;
+    const LinkRef<R> none{};
+    const typename Cd::T* fin = sub_pop(wait_previous(f_prev), first);
+    typename Cd::T* out = sub_pop(fout, first);
+    double acc = 0.0;
+    if (live) {
+        R F[19];
+        LinkGather<STORE, false>::all(F, fin, L, K, n, none);
+        R r = F[0];
 #pragma unroll
-            for (int s = 1; s < 19; ++s) r = r + F[s];
-            const R rho = Cd::DEV ? (R)1 + r : r;
-            R vx = vsum<0>(F) / rho, vy = vsum<1>(F) / rho, vz = vsum<2>(F) / rho;
-            if constexpr (FORCE) {
-                vx = vx + C.fhalf[0] / rho;
-                vy = vy + C.fhalf[1] / rho;
-                vz = vz + C.fhalf[2] / rho;
-            }
-            if constexpr (CHECK) acc += (double)vx;
-            collide_sp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, C);
-            store_node<STORE>(F, sfout, n, (R)0, seed);
+        for (int s = 1; s < 19; ++s) r = r + F[s];
+        const R rho = Cd::DEV ? (R)1 + r : r;
+        R vx = vsum<0>(F) / rho, vy = vsum<1>(F) / rho, vz = vsum<2>(F) / rho;
+        if constexpr (FORCE) {
+            vx = vx + C.fhalf[0] / rho;
+            vy = vy + C.fhalf[1] / rho;
+            vz = vz + C.fhalf[2] / rho;
         }
-        if constexpr (CHECK) {
-            for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
-            if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                double s = 0.0;
-                for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += s_red[w];
-                partial[t] = s;
-            }
-            __syncthreads();
+        if constexpr (CHECK) acc += (double)vx;
+        collide_sp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, C);
+        store_node<STORE>(F, out, n, (R)0, seed);
+    }
+    if constexpr (CHECK) {
+        for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);
+        if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double s = 0.0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += s_red[w];
+            partial[blockIdx.x] = s;
         }
     }
 }
@@ -198,10 +187,20 @@ int launch_one(LbmBatch* b, int k, bool check, cudaStream_t s) {
     const int cur = k & 1;
     const T* fin = (const T*)h->d_f[cur];
     T* fout = (T*)h->d_f[cur ^ 1];
-    int32_t* ctr = b->d_counters + k;
+    if (b->tiles.empty()) return LBM_OK;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)b->tiles.size());
+    cfg.blockDim = dim3((unsigned)b->block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = k > 0 ? 1 : 0;   // the first step of a group waits for the seed in stream order
+    cudaError_t e = cudaSuccess;
     auto args = [&](auto kern) {
-        kern<<<b->grid, b->block, 0, s>>>(C, b->d_subs, b->d_tiles, b->d_ntiles, ctr, fin, fout, h->d_map, h->d_coord,
-                                          seed_base(b), b->d_partial);
+        e = cudaLaunchKernelEx(&cfg, kern, C, (const BatchTile*)b->d_tiles, fin, fout, h->links,
+                               (const uint32_t*)b->d_seed, b->d_partial);
     };
     if (h->force) {
         if (check) args(batch_step_kernel<STORE, true, true>);
@@ -210,7 +209,7 @@ int launch_one(LbmBatch* b, int k, bool check, cudaStream_t s) {
         if (check) args(batch_step_kernel<STORE, false, true>);
         else args(batch_step_kernel<STORE, false, false>);
     }
-    return lbm_cuda_check(h, cudaGetLastError(), "batch_step_kernel launch");
+    return lbm_cuda_check(h, e != cudaSuccess ? e : cudaGetLastError(), "batch_step_kernel launch");
 }
 
 int launch_dispatch(LbmBatch* b, int k, bool check, cudaStream_t s) {
@@ -220,25 +219,6 @@ int launch_dispatch(LbmBatch* b, int k, bool check, cudaStream_t s) {
     case LBM_STORE_BF16_DEV: return launch_one<LBM_STORE_BF16_DEV>(b, k, check, s);
     case LBM_STORE_F32_DEV: return launch_one<LBM_STORE_F32_DEV>(b, k, check, s);
     case LBM_STORE_F64: return launch_one<LBM_STORE_F64>(b, k, check, s);
-    }
-    return batch_err(b, LBM_EINVAL, "unknown storage");
-}
-
-template <int STORE>
-int occupancy(LbmBatch* b, int* per_sm) {
-    // the CHECK variant has the same resource use; ask the runtime for the unforced and forced kernels
-    const void* k = b->h.force ? (const void*)batch_step_kernel<STORE, true, false>
-                               : (const void*)batch_step_kernel<STORE, false, false>;
-    return lbm_cuda_check(&b->h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k, b->block, 0), "occupancy");
-}
-
-int occ_dispatch(LbmBatch* b, int* per_sm) {
-    switch (b->h.p.storage) {
-    case LBM_STORE_F32: return occupancy<LBM_STORE_F32>(b, per_sm);
-    case LBM_STORE_F16_DEV: return occupancy<LBM_STORE_F16_DEV>(b, per_sm);
-    case LBM_STORE_BF16_DEV: return occupancy<LBM_STORE_BF16_DEV>(b, per_sm);
-    case LBM_STORE_F32_DEV: return occupancy<LBM_STORE_F32_DEV>(b, per_sm);
-    case LBM_STORE_F64: return occupancy<LBM_STORE_F64>(b, per_sm);
     }
     return batch_err(b, LBM_EINVAL, "unknown storage");
 }
@@ -271,29 +251,29 @@ int macros_t(LbmBatch* b, int q, float* d_out) {
     return lbm_cuda_check(h, cudaGetLastError(), "batch_macros_kernel launch");
 }
 
+void destroy_graph(LbmBatch* b) {
+    if (b->graph) cudaGraphExecDestroy(b->graph);
+    b->graph = nullptr;
+    b->graph_steps = 0;
+}
+
 int rebuild_tiles(LbmBatch* b) {
     b->tiles.clear();
     for (size_t q = 0; q < b->subs.size(); ++q) {
         if (!b->active[q]) continue;
         const BatchSub& s = b->subs[q];
-        const int len = std::max(32, b->tile_len[q]);
+        const int len = std::min((std::max(32, b->tile_len[q]) + 31) / 32 * 32, b->block);   // whole link groups
         for (int a = 0; a < s.n_fluid; a += len)
-            b->tiles.push_back({(int32_t)q, a, std::min(s.n_fluid, a + len), 0});
+            b->tiles.push_back({(int32_t)(s.node_begin / 32), a, std::min(s.n_fluid, a + len), (int32_t)q});
     }
     LbmHandle* h = &b->h;
+    destroy_graph(b);   // its grids are the tile count
     if ((int64_t)b->tiles.size() > b->max_tiles) return batch_err(b, LBM_EINVAL, "tile list exceeds its allocation");
     const int32_t nt = (int32_t)b->tiles.size();
     int rc = 0;
     if (nt) rc = lbm_cuda_check(h, cudaMemcpyAsync(b->d_tiles, b->tiles.data(), sizeof(BatchTile) * nt, cudaMemcpyHostToDevice, h->stream), "copy tiles");
-    if (!rc) rc = lbm_cuda_check(h, cudaMemcpyAsync(b->d_ntiles, &nt, sizeof(int32_t), cudaMemcpyHostToDevice, h->stream), "copy ntiles");
     if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "rebuild tiles");
     return rc;
-}
-
-void destroy_graph(LbmBatch* b) {
-    if (b->graph) cudaGraphExecDestroy(b->graph);
-    b->graph = nullptr;
-    b->graph_steps = 0;
 }
 
 // Capture `nsteps` steps (the last one writes the per-tile partials) into a graph.
@@ -303,7 +283,6 @@ int capture(LbmBatch* b, int32_t nsteps) {
     cudaGraph_t g;
     int rc = lbm_cuda_check(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     if (rc) return rc;
-    cudaMemsetAsync(b->d_counters, 0, sizeof(int32_t) * nsteps, h->stream);
     for (int k = 0; k < nsteps && !rc; ++k) rc = launch_dispatch(b, k, k == nsteps - 1, h->stream);
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (rc) return rc;
@@ -377,7 +356,7 @@ int lbm_batch_create(const LbmParams* params, int32_t n_sub, const int32_t* dims
     coord.resize(h->np, 0);
     h->ncell = cells;
     b->active.assign(n_sub, 1);
-    b->tile_len.assign(n_sub, 1024);
+    b->tile_len.assign(n_sub, 128);
     b->steps.assign(n_sub, 0);
     b->max_tiles = 0;
     for (auto& s : b->subs) b->max_tiles += (s.n_fluid + 31) / 32;   // tiles of >= 32 nodes
@@ -392,12 +371,12 @@ int lbm_batch_create(const LbmParams* params, int32_t n_sub, const int32_t* dims
     alloc(&h->d_f[1], h->elem * 19 * h->np);
     alloc((void**)&b->d_subs, sizeof(BatchSub) * n_sub);
     alloc((void**)&b->d_tiles, sizeof(BatchTile) * b->max_tiles);
-    alloc((void**)&b->d_ntiles, sizeof(int32_t));
     alloc((void**)&b->d_partial, sizeof(double) * b->max_tiles);
-    alloc((void**)&b->d_counters, sizeof(int32_t) * (4096 + 4));   // + the first step of the launch group
+    alloc((void**)&b->d_seed, sizeof(uint32_t));
     if (!rc) rc = lbm_cuda_check(h, cudaMemcpy(h->d_map, map.data(), sizeof(int32_t) * map.size(), cudaMemcpyHostToDevice), "copy map");
     if (!rc) rc = lbm_cuda_check(h, cudaMemcpy(h->d_coord, coord.data(), sizeof(uint32_t) * h->np, cudaMemcpyHostToDevice), "copy coord");
     if (!rc) rc = lbm_cuda_check(h, cudaMemcpy(b->d_subs, b->subs.data(), sizeof(BatchSub) * n_sub, cudaMemcpyHostToDevice), "copy subs");
+    if (!rc) rc = links_build(h, b->subs.data(), n_sub);
     if (rc) { lbm_batch_destroy(b); return rc; }
     h->have_geometry = true;
     *out = b;
@@ -412,9 +391,9 @@ int lbm_batch_destroy(LbmBatch* b) {
     destroy_graph(b);
     cudaFree(b->d_subs);
     cudaFree(b->d_tiles);
-    cudaFree(b->d_ntiles);
     cudaFree(b->d_partial);
-    cudaFree(b->d_counters);
+    cudaFree(b->d_seed);
+    cudaFree(h->d_links);
     cudaFree(h->d_map);
     cudaFree(h->d_coord);
     cudaFree(h->d_f[0]);
@@ -424,7 +403,7 @@ int lbm_batch_destroy(LbmBatch* b) {
     return LBM_OK;
 }
 
-// Tile length (nodes) per subvolume and threads per CTA of the persistent kernel.
+// Threads per CTA, and the nodes of a CTA's tile per subvolume: whole link groups of 32, at most its threads.
 int lbm_batch_configure(LbmBatch* b, const int32_t* tile_len, int32_t block) {
     if (!b || !tile_len) return lbm_set_err(nullptr, LBM_EINVAL, "lbm_batch_configure: NULL argument");
     if (block < 64 || block > 256 || block % 32) return batch_err(b, LBM_EINVAL, "lbm_batch_configure: block must be 64..256, multiple of 32");
@@ -441,10 +420,7 @@ int lbm_batch_init(LbmBatch* b) {
     if (!b) return lbm_set_err(nullptr, LBM_EINVAL, "lbm_batch_init: NULL");
     LbmHandle* h = &b->h;
     cudaSetDevice(h->device);
-    int per_sm = 0;
-    int rc = occ_dispatch(b, &per_sm);
-    if (rc) return rc;
-    b->grid = std::max(1, per_sm) * h->sm_count;
+    int rc = LBM_OK;
     std::fill(b->active.begin(), b->active.end(), (uint8_t)1);
     std::fill(b->steps.begin(), b->steps.end(), (int64_t)0);
     switch (h->p.storage) {
@@ -466,7 +442,7 @@ int lbm_batch_init(LbmBatch* b) {
 static int set_seed_base(LbmBatch* b, int32_t chunk) {
     const uint32_t v = b->seed_step;
     b->seed_step += (uint32_t)chunk;
-    return lbm_cuda_check(&b->h, cudaMemcpyAsync(b->d_counters + 4096, &v, sizeof(v), cudaMemcpyHostToDevice, b->h.stream),
+    return lbm_cuda_check(&b->h, cudaMemcpyAsync(b->d_seed, &v, sizeof(v), cudaMemcpyHostToDevice, b->h.stream),
                           "seed base");
 }
 
@@ -489,7 +465,6 @@ static int batch_run(LbmBatch* b, int32_t nsteps, int32_t chunk, int32_t use_gra
     }
     for (int32_t done = 0; done < nsteps; done += chunk) {
         int rc = set_seed_base(b, chunk);
-        if (!rc) rc = lbm_cuda_check(h, cudaMemsetAsync(b->d_counters, 0, sizeof(int32_t) * chunk, h->stream), "counters");
         for (int k = 0; k < chunk && !rc; ++k) rc = launch_dispatch(b, k, k == chunk - 1, h->stream);
         if (rc) return rc;
     }
@@ -630,7 +605,7 @@ int lbm_batch_info(LbmBatch* b, int64_t* n_nodes, int64_t* n_fluid, int32_t* gri
     for (auto& s : b->subs) nf += s.n_fluid;
     if (n_nodes) *n_nodes = b->h.n_fluid;
     if (n_fluid) *n_fluid = nf;
-    if (grid) *grid = b->grid;
+    if (grid) *grid = (int32_t)b->tiles.size();
     if (n_tiles) *n_tiles = (int32_t)b->tiles.size();
     return LBM_OK;
 }

@@ -260,7 +260,10 @@ int lbm_set_geometry_strided(LbmHandle* h, const int8_t* solid, int64_t si, int6
     h->have_geometry = h->initialized = h->macros_valid = false;
     int rc = geom_build(h, solid, si, sj, sk);
     if (!rc) rc = sp_tiles_setup(h);
-    if (!rc && !h->f64 && !h->p.two_phase) rc = links_build(h);
+    if (!rc && !h->f64 && !h->p.two_phase) {
+        const LbmLinkLattice lat{h->p.nx, h->p.ny, h->p.nz, h->n_fluid, 0, 0};
+        rc = links_build(h, &lat, 1);
+    }
     if (rc) { free_lattice(h); return rc; }
     const size_t rbytes = h->f64 ? 8 : 4;
     rc = rc ? rc : dev_alloc(h, &h->d_f[0], h->elem * 19 * h->np, "f_A");

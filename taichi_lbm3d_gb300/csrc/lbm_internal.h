@@ -111,8 +111,8 @@ int lbm_cuda_check(LbmHandle* h, cudaError_t e, const char* what);
 // index construction and dense output (lbm_geom.cu)
 int geom_build(LbmHandle* h, const int8_t* solid, int64_t si, int64_t sj, int64_t sk);
 int geom_host_index(LbmHandle* h);
-// Neighbour links of the index (lbm_links.cu).
-int links_build(LbmHandle* h);
+// Neighbour links (lbm_links.cu).
+int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count);
 template <typename O>
 int geom_dense_out(LbmHandle* h, const void* dsrc, int comps, O* out, O fill);
 

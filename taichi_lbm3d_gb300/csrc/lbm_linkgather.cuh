@@ -22,6 +22,7 @@ __device__ __forceinline__ const T* wait_previous(const T* p) {
 struct NodeLinks {
     int4 a, b;          // the group's row starts
     uint32_t w, bits;
+    int lane;           // place in the group
     __device__ __forceinline__ void load(const LbmLinks& L, int n) {
         const int4* head = reinterpret_cast<const int4*>(L.head + n / LBM_LINK_GROUP);
         a = __ldg(head);
@@ -29,6 +30,7 @@ struct NodeLinks {
         const uint2 x = __ldg(L.node + n);
         w = x.x;
         bits = x.y;
+        lane = n & (LBM_LINK_GROUP - 1);
     }
     // Node across in row r.
     template <int RW>
@@ -36,7 +38,7 @@ struct NodeLinks {
         const int4& h = RW < 4 ? a : b;
         const int start = (RW & 3) == 0 ? h.x : (RW & 3) == 1 ? h.y : (RW & 3) == 2 ? h.z : h.w;
         const uint32_t q = RW < 6 ? w >> (5 * RW) & 31u : bits >> (22 + 5 * (RW - 6)) & 31u;
-        return start + (int)(threadIdx.x & 31) + (int)q;
+        return start + lane + (int)q;
     }
 };
 
@@ -46,6 +48,7 @@ struct NodeLinks {
 template <typename R>
 struct LinkRef {
     R at, xm, xp;
+    LinkRef() = default;
     __device__ __forceinline__ LinkRef(const LbmRef<R>& ref, int i, int nx) {
         const bool inside = __all_sync(__activemask(), i > 0 && i < nx - 1);
         at = lbm_ref_at(ref, i);

@@ -142,17 +142,22 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
 
 }  // namespace
 
-// Links of the lattice whose map and coordinates are on the device; one
-// allocation (h->d_links).  Records: room for every node of the periodic faces;
-// a geometry that needs more (rows far from a line) gets a second one.
-int links_build(LbmHandle* h) {
+// Links of `count` lattices whose maps and coordinates lie in h->d_map and
+// h->d_coord (node numbers local to each lattice); one allocation
+// (h->d_links).  Records: room for every node of the periodic faces; geometries
+// that need more (rows far from a line) get a second one.
+int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
     const LbmParams& p = h->p;
     const int64_t ngroup = h->np / LBM_LINK_GROUP;
-    int64_t cap = 0;
-    const int64_t area[3] = {(int64_t)p.ny * p.nz, (int64_t)p.nx * p.nz, (int64_t)p.nx * p.ny};
-    for (int f = 0; f < 6; ++f)
-        if (p.bc[f] == LBM_BC_PERIODIC || (p.bc[f] == LBM_BC_VELOCITY && p.bc_form != 0)) cap += area[f / 2];
-    cap = std::min<int64_t>(cap, h->n_fluid) + h->n_fluid / 512 + 32;
+    int64_t cap = 32;
+    for (int q = 0; q < count; ++q) {
+        const LbmLinkLattice& l = lat[q];
+        const int64_t area[3] = {(int64_t)l.ny * l.nz, (int64_t)l.nx * l.nz, (int64_t)l.nx * l.ny};
+        int64_t seam = 0;
+        for (int f = 0; f < 6; ++f)
+            if (p.bc[f] == LBM_BC_PERIODIC || (p.bc[f] == LBM_BC_VELOCITY && p.bc_form != 0)) seam += area[f / 2];
+        cap += std::min<int64_t>(seam, l.n_fluid) + l.n_fluid / 512;
+    }
     for (;;) {
         const size_t node = sizeof(uint2) * h->np, head = sizeof(LbmLinkHead) * ngroup;
         const size_t rec0 = (sizeof(int32_t) * (ngroup + 1) + 15) / 16 * 16;   // + the count
@@ -164,28 +169,36 @@ int links_build(LbmHandle* h) {
         }
         h->device_bytes += (int64_t)bytes;
         char* at = (char*)h->d_links;
-        LinkBuild B{};
-        B.map = h->d_map;
-        B.coord = h->d_coord;
-        B.nx = p.nx; B.ny = p.ny; B.nz = p.nz;
-        B.n_fluid = h->n_fluid;
-        for (int f = 0; f < 6; ++f) B.bc[f] = p.bc[f];
-        B.bc_form = p.bc_form;
-        B.node = (uint2*)at;
-        B.head = (LbmLinkHead*)(at + node);
-        B.rec0 = (int32_t*)(at + node + head);
-        B.total = B.rec0 + ngroup;
-        B.rec = (int32_t*)(at + node + head + rec0);
-        B.cap = (int32_t)cap;
-        h->links = {B.node, B.head, B.rec0, B.rec};
-        rc = lbm_cuda_check(h, cudaMemsetAsync(B.total, 0, sizeof(int32_t), h->stream), "link records");
+        const LbmLinks L{(uint2*)at, (LbmLinkHead*)(at + node), (int32_t*)(at + node + head), (int32_t*)(at + node + head + rec0)};
+        h->links = L;
+        int32_t* d_total = (int32_t*)(at + node + head) + ngroup;
+        rc = lbm_cuda_check(h, cudaMemsetAsync(d_total, 0, sizeof(int32_t), h->stream), "link records");
         if (rc) return rc;
-        const int grid = (int)((ngroup + 3) / 4);
-        link_build_kernel<false><<<grid, 128, 0, h->stream>>>(B, (int)ngroup);
-        link_build_kernel<true><<<grid, 128, 0, h->stream>>>(B, (int)ngroup);
+        for (int pass = 0; pass < 2; ++pass)
+            for (int q = 0; q < count; ++q) {
+                const LbmLinkLattice& l = lat[q];
+                LinkBuild B{};
+                B.map = h->d_map + l.map_off;
+                B.coord = h->d_coord + l.node_begin;
+                B.nx = l.nx; B.ny = l.ny; B.nz = l.nz;
+                B.n_fluid = l.n_fluid;
+                for (int f = 0; f < 6; ++f) B.bc[f] = p.bc[f];
+                B.bc_form = p.bc_form;
+                B.node = (uint2*)L.node + l.node_begin;
+                B.head = (LbmLinkHead*)L.head + l.node_begin / LBM_LINK_GROUP;
+                B.rec0 = (int32_t*)L.rec0 + l.node_begin / LBM_LINK_GROUP;
+                B.rec = (int32_t*)L.rec;
+                B.cap = (int32_t)cap;
+                B.total = d_total;
+                // a lone lattice fills the padding of its arrays too (at most 64 nodes)
+                const int groups = count == 1 ? (int)ngroup : (l.n_fluid + LBM_LINK_GROUP - 1) / LBM_LINK_GROUP;
+                if (!groups) continue;
+                if (pass == 0) link_build_kernel<false><<<(groups + 3) / 4, 128, 0, h->stream>>>(B, groups);
+                else link_build_kernel<true><<<(groups + 3) / 4, 128, 0, h->stream>>>(B, groups);
+            }
         rc = lbm_cuda_check(h, cudaGetLastError(), "link_build_kernel launch");
         int32_t total = 0;
-        if (!rc) rc = lbm_cuda_check(h, cudaMemcpyAsync(&total, B.total, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream), "link records");
+        if (!rc) rc = lbm_cuda_check(h, cudaMemcpyAsync(&total, d_total, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream), "link records");
         if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "neighbour links");
         if (rc || total <= cap) return rc;
         cudaFree(h->d_links);

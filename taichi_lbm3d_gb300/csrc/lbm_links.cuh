@@ -43,6 +43,13 @@ struct LbmLinks {
     const int32_t* rec;           // LBM_LINK_REC per record
 };
 
+// A lattice among those whose links are built together.
+struct LbmLinkLattice {
+    int32_t nx, ny, nz, n_fluid;
+    int64_t map_off;      // first cell of its map
+    int64_t node_begin;   // first node (a multiple of 32)
+};
+
 // (e_y, e_z) of row r: rows 0..3 hold three directions each, 4..7 one.
 __host__ __device__ constexpr int lbm_link_ey(int r) {
     return (r == 0 || r == 4 || r == 6) ? 1 : (r == 1 || r == 5 || r == 7) ? -1 : 0;

@@ -118,10 +118,11 @@ void free_lattice(LbmHandle* h) {
     dev_free(h->d_rho);
     dev_free(h->d_v);
     dev_free(h->d_psi);
-    dev_free(h->d_rr[0]);
-    dev_free(h->d_rr[1]);
-    dev_free(h->d_rb[0]);
-    dev_free(h->d_rb[1]);
+    dev_free(h->d_psi0);
+    dev_free(h->d_rr);
+    dev_free(h->d_rb);
+    dev_free(h->d_crec);
+    dev_free(h->d_pull_vz);
     dev_free(h->d_cs);
     dev_free(h->d_ns);
     dev_free(h->d_gstale);
@@ -260,7 +261,7 @@ int lbm_set_geometry_strided(LbmHandle* h, const int8_t* solid, int64_t si, int6
     h->have_geometry = h->initialized = h->macros_valid = false;
     int rc = geom_build(h, solid, si, sj, sk);
     if (!rc) rc = sp_tiles_setup(h);
-    if (!rc && !h->f64 && !h->p.two_phase) {
+    if (!rc && (!h->f64 || h->p.two_phase)) {
         const LbmLinkLattice lat{h->p.nx, h->p.ny, h->p.nz, h->n_fluid, 0, 0};
         rc = links_build(h, &lat, 1);
     }
@@ -273,10 +274,11 @@ int lbm_set_geometry_strided(LbmHandle* h, const int8_t* solid, int64_t si, int6
     rc = rc ? rc : dev_alloc(h, &h->d_v, rbytes * 3 * h->np, "v");
     if (!rc && h->p.two_phase) {
         rc = rc ? rc : dev_alloc(h, &h->d_psi, rbytes * h->np, "psi");
-        rc = rc ? rc : dev_alloc(h, &h->d_rr[0], rbytes * h->np, "rho_r A");
-        rc = rc ? rc : dev_alloc(h, &h->d_rr[1], rbytes * h->np, "rho_r B");
-        rc = rc ? rc : dev_alloc(h, &h->d_rb[0], rbytes * h->np, "rho_b A");
-        rc = rc ? rc : dev_alloc(h, &h->d_rb[1], rbytes * h->np, "rho_b B");
+        rc = rc ? rc : dev_alloc(h, &h->d_psi0, sizeof(float) * h->ncell, "initial psi");
+        rc = rc ? rc : dev_alloc(h, &h->d_rr, rbytes * h->np, "rho_r");
+        rc = rc ? rc : dev_alloc(h, &h->d_rb, rbytes * h->np, "rho_b");
+        rc = rc ? rc : dev_alloc(h, &h->d_crec, rbytes * 4 * h->np, "colour records");
+        rc = rc ? rc : dev_alloc(h, &h->d_pull_vz, rbytes * h->np, "pulled v_z");
         rc = rc ? rc : dev_alloc(h, &h->d_cs, rbytes * 9 * h->np, "recolouring amounts");
     }
     h->red_blocks = (int)std::min<int64_t>(4 * h->sm_count, (h->n_fluid + 255) / 256 + 1);
@@ -292,7 +294,7 @@ int lbm_set_geometry_strided(LbmHandle* h, const int8_t* solid, int64_t si, int6
     h->have_psi = false;
     // the link steps do not read the map; a window that nothing uses costs the
     // populations that part of L2 (256^3 pack: 200 us a step with it, 165 without)
-    if (h->f64 || h->p.two_phase || h->tiled) l2_persist_map(h);
+    if (!h->p.two_phase && (h->f64 || h->tiled)) l2_persist_map(h);
     return LBM_OK;
 }
 
@@ -345,7 +347,10 @@ int lbm_set_psi(LbmHandle* h, const float* psi) {
     if (!h || !psi) return lbm_set_err(h, LBM_EINVAL, "lbm_set_psi: NULL argument");
     if (!h->p.two_phase) return lbm_set_err(h, LBM_ESTATE, "lbm_set_psi: handle is single phase");
     if (!h->have_geometry) return lbm_set_err(h, LBM_ESTATE, "lbm_set_psi: call lbm_set_geometry first");
-    h->psi0.assign(psi, psi + h->ncell);
+    cudaSetDevice(h->device);
+    int rc = lbm_cuda_check(h, cudaMemcpyAsync(h->d_psi0, psi, sizeof(float) * h->ncell, cudaMemcpyHostToDevice, h->stream), "copy psi");
+    if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "copy psi");
+    if (rc) return rc;
     h->have_psi = true;
     h->initialized = false;
     return LBM_OK;
@@ -494,15 +499,11 @@ int lbm_get_phase(LbmHandle* h, float* psi, float* rho_r, float* rho_b) {
     cudaSetDevice(h->device);
     int rc = LBM_OK;
     if (psi) {
-        // fluid cells from the device; solid cells keep the input psi (the reference never updates them)
-        std::vector<float> fl(h->ncell);
-        rc = geom_host_index(h);
-        if (!rc) rc = scatter_dense<float>(h, h->d_psi, 1, fl.data(), 0.0f);
-        if (!rc)
-            for (int64_t c = 0; c < h->ncell; ++c) psi[c] = h->solid[c] ? h->psi0[c] : fl[c];
+        // solid cells keep the input psi (the reference never updates them)
+        rc = geom_dense_out<float>(h, h->d_psi, 1, psi, 0.0f, h->d_psi0);
     }
-    if (!rc && rho_r) rc = scatter_dense<float>(h, h->d_rr[h->ccur], 1, rho_r, 0.0f);
-    if (!rc && rho_b) rc = scatter_dense<float>(h, h->d_rb[h->ccur], 1, rho_b, 0.0f);
+    if (!rc && rho_r) rc = scatter_dense<float>(h, h->d_rr, 1, rho_r, 0.0f);
+    if (!rc && rho_b) rc = scatter_dense<float>(h, h->d_rb, 1, rho_b, 0.0f);
     return rc;
 }
 

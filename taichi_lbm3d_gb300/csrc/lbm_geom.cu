@@ -127,13 +127,14 @@ __global__ void __launch_bounds__(GEO_THREADS) geo_write_kernel(const MaskView m
     }
 }
 
-// out[c*comps + d] = node value d of cell c, or fill for solid cells.
+// out[c*comps + d] = node value d of cell c, or fill (fill_cells[c] where given) for solid cells.
 template <typename S, typename O>
 __global__ void dense_out_kernel(const int32_t* __restrict__ map, const S* __restrict__ src, int64_t np, int comps,
-                                 int64_t ncell, O fill, O* __restrict__ out) {
+                                 int64_t ncell, O fill, const O* __restrict__ fill_cells, O* __restrict__ out) {
     const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= ncell) return;
     const int32_t n = map[c];
+    if (n < 0 && fill_cells) fill = fill_cells[c];
     for (int d = 0; d < comps; ++d) out[c * comps + d] = n >= 0 ? (O)src[d * np + n] : fill;
 }
 }  // namespace
@@ -212,21 +213,21 @@ int geom_host_index(LbmHandle* h) {
 // Dense host array (comps interleaved per cell) from a node-ordered device
 // array (comps components of stride np, the handle's compute type).
 template <typename O>
-int geom_dense_out(LbmHandle* h, const void* dsrc, int comps, O* out, O fill) {
+int geom_dense_out(LbmHandle* h, const void* dsrc, int comps, O* out, O fill, const O* fill_cells) {
     const int64_t n = h->ncell * comps;
     O* d_out = nullptr;
     int rc = lbm_cuda_check(h, cudaMallocAsync((void**)&d_out, sizeof(O) * n, h->stream), "output staging");
     if (rc) return rc;
     const int blocks = (int)((h->ncell + 255) / 256);
     if (h->f64)
-        dense_out_kernel<double, O><<<blocks, 256, 0, h->stream>>>(h->d_map, (const double*)dsrc, h->np, comps, h->ncell, fill, d_out);
+        dense_out_kernel<double, O><<<blocks, 256, 0, h->stream>>>(h->d_map, (const double*)dsrc, h->np, comps, h->ncell, fill, fill_cells, d_out);
     else
-        dense_out_kernel<float, O><<<blocks, 256, 0, h->stream>>>(h->d_map, (const float*)dsrc, h->np, comps, h->ncell, fill, d_out);
+        dense_out_kernel<float, O><<<blocks, 256, 0, h->stream>>>(h->d_map, (const float*)dsrc, h->np, comps, h->ncell, fill, fill_cells, d_out);
     rc = lbm_cuda_check(h, cudaGetLastError(), "dense_out_kernel launch");
     if (!rc) rc = lbm_cuda_check(h, cudaMemcpyAsync(out, d_out, sizeof(O) * n, cudaMemcpyDeviceToHost, h->stream), "copy out");
     cudaFreeAsync(d_out, h->stream);
     if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "copy out");
     return rc;
 }
-template int geom_dense_out<float>(LbmHandle*, const void*, int, float*, float);
-template int geom_dense_out<double>(LbmHandle*, const void*, int, double*, double);
+template int geom_dense_out<float>(LbmHandle*, const void*, int, float*, float, const float*);
+template int geom_dense_out<double>(LbmHandle*, const void*, int, double*, double, const double*);

@@ -70,7 +70,6 @@ struct LbmHandle {
     std::vector<int32_t> cell_of_node;     // n_fluid (made on demand)
     bool host_index_valid = false;
     bool l2_persist = false;               // the map is this stream's persisting L2 window
-    std::vector<float> psi0;               // dense initial psi (two phase)
 
     int32_t* d_map = nullptr;              // dense: node index or -1 (solid); LBM_MAP_PAD extra -1 entries
     int2* d_tinfo = nullptr;               // staged step: per 256-node tile, first staged row and plane/rows
@@ -89,10 +88,12 @@ struct LbmHandle {
     void* d_v = nullptr;                   // [3][np]
     // two phase
     void* d_psi = nullptr;                 // [np] psi at fluid nodes
-    void* d_rr[2] = {nullptr, nullptr};    // rho_r, double-buffered [np]
-    void* d_rb[2] = {nullptr, nullptr};    // rho_b
+    float* d_psi0 = nullptr;               // dense initial psi
+    void* d_rr = nullptr;                  // rho_r [np]
+    void* d_rb = nullptr;                  // rho_b [np]
+    void* d_crec = nullptr;                // what the colour launch pulls of a node: (rho_r, rho_b, v_x, v_y) [np][4]
+    void* d_pull_vz = nullptr;             // and v_z [np]
     void* d_cs = nullptr;                  // recolouring amounts of the 9 pairs [9][np]
-    int ccur = 0;
     // grey scale (partial bounce-back)
     bool grey = false;
     void* d_ns = nullptr;                  // [np] grey value per node (compute type)
@@ -114,7 +115,7 @@ int geom_host_index(LbmHandle* h);
 // Neighbour links (lbm_links.cu).
 int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count);
 template <typename O>
-int geom_dense_out(LbmHandle* h, const void* dsrc, int comps, O* out, O fill);
+int geom_dense_out(LbmHandle* h, const void* dsrc, int comps, O* out, O fill, const O* fill_cells = nullptr);
 
 // single phase (lbm_sp.cu)
 int sp_launch_init(LbmHandle* h, const void* rho_nodes, const void* v_nodes);

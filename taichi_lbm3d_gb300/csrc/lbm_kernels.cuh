@@ -246,6 +246,50 @@ __device__ __forceinline__ R vsum(const R* F) {
     return a;
 }
 
+// Quotients of K numbers by one divisor, correctly rounded.  FP32: with y the
+// correctly rounded reciprocal, q = a y followed by q + y (a - q b) in fused
+// operations is the correctly rounded a / b (Markstein, IBM J. Res. Dev. 34,
+// 1990), away from underflow of the residual: one reciprocal and three
+// operations a quotient.  A divisor outside the range where that is sure (a
+// lattice that has diverged) takes the division itself.
+template <int K>
+__device__ __forceinline__ void quotients(float (&a)[K], float b) {
+    if (b > 1e-12f && b < 1e12f) {
+        const float y = __frcp_rn(b);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const float q = a[k] * y;
+            a[k] = lbm_fma<float>(lbm_fma<float>(-q, b, a[k]), y, q);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) a[k] = a[k] / b;
+    }
+}
+template <int K>
+__device__ __forceinline__ void quotients(double (&a)[K], double b) {
+#pragma unroll
+    for (int k = 0; k < K; ++k) a[k] = a[k] / b;
+}
+
+// v = j / rho, plus half the body force over rho (SP:382-388).
+template <typename R, bool FORCE>
+__device__ __forceinline__ void velocity(R& vx, R& vy, R& vz, R rho, const SpConsts<R>& C) {
+    if constexpr (FORCE) {
+        R q[6] = {vx, vy, vz, C.fhalf[0], C.fhalf[1], C.fhalf[2]};
+        quotients(q, rho);
+        vx = q[0] + q[3];
+        vy = q[1] + q[4];
+        vz = q[2] + q[5];
+    } else {
+        R q[3] = {vx, vy, vz};
+        quotients(q, rho);
+        vx = q[0];
+        vy = q[1];
+        vz = q[2];
+    }
+}
+
 // Class collision (SP:222-241): F, rho, v -> f (in place).  In deviation form
 // F holds f - w and r is rho - 1 (moment 0 of M (f - w)).
 // FAST (deviation-form kernels): pair-form transforms and FMA relaxation; the

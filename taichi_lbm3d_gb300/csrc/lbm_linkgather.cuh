@@ -18,6 +18,13 @@ __device__ __forceinline__ const T* wait_previous(const T* p) {
     return p;
 }
 
+// The same for a second pointer, after the wait.
+template <typename T>
+__device__ __forceinline__ const T* launder(const T* p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return p;
+}
+
 // A node's links: loaded before the wait (they never change between steps).
 struct NodeLinks {
     int4 a, b;          // the group's row starts
@@ -39,6 +46,28 @@ struct NodeLinks {
         const int start = (RW & 3) == 0 ? h.x : (RW & 3) == 1 ? h.y : (RW & 3) == 2 ? h.z : h.w;
         const uint32_t q = RW < 6 ? w >> (5 * RW) & 31u : bits >> (22 + 5 * (RW - 6)) & 31u;
         return start + lane + (int)q;
+    }
+    // Pull source of direction S of node n (where its bit is clear).
+    template <int S>
+    __device__ __forceinline__ int source(int n) const {
+        constexpr int ex = lbm_ex(S), ey = lbm_ey(S), ez = lbm_ez(S);
+        if constexpr (ey == 0 && ez == 0) {
+            return n - ex;
+        } else {
+            constexpr int rw = lbm_link_row(ey, ez);
+            if constexpr (ex > 0) return rank<rw>() - 1;
+            // x + 1 ranks after x only where x itself is fluid
+            if constexpr (ex < 0) return rank<rw>() + (int)(~bits >> lbm_link_dir(rw, 0) & 1u);
+            return rank<rw>();
+        }
+    }
+    // Whether any node of the warp (one group) has a record; this node's.
+    __device__ __forceinline__ bool record(const LbmLinks& L, int n, const int32_t*& rec) const {
+        const uint32_t e = __ballot_sync(__activemask(), bits & LBM_LINK_EXC);
+        if (e)
+            rec = L.rec + (int64_t)LBM_LINK_REC *
+                              (__ldg(L.rec0 + n / LBM_LINK_GROUP) + __popc(e & ((1u << (threadIdx.x & 31)) - 1u)));
+        return e != 0;
     }
 };
 
@@ -70,31 +99,18 @@ struct LinkGather {
     using T = typename Cd::T;
     using R = typename Cd::R;
     template <int S>
-    static __device__ __forceinline__ void one(R* F, const T* fin, int own, int src, uint32_t bits, const LinkRef<R>& rx) {
-        const bool bounce = bits >> S & 1u;
-        const int a = bounce ? own + 32 * (lbm_lr(S) - S) : lbm_eoff32(src);
+    static __device__ __forceinline__ void one(R* F, const T* fin, int own, const NodeLinks& K, int n, const LinkRef<R>& rx) {
+        const bool bounce = K.bits >> S & 1u;
+        const int a = bounce ? own + 32 * (lbm_lr(S) - S) : lbm_eoff32(K.template source<S>(n));
         F[S] = Cd::template dec<S>(fin[a + 32 * S]);
         if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), bounce ? rx.at : rx.template of<S>(), F[S]);
     }
-    template <int RW>
-    static __device__ __forceinline__ void row(R* F, const T* fin, int own, const NodeLinks& K, const LinkRef<R>& rx) {
-        constexpr int c = lbm_link_dir(RW, 0);
-        const int m = K.template rank<RW>();
-        one<c>(F, fin, own, m, K.bits, rx);
-        if constexpr (RW < 4) {
-            one<lbm_link_dir(RW, 1)>(F, fin, own, m - 1, K.bits, rx);
-            // x + 1 ranks after x only where x itself is fluid
-            one<lbm_link_dir(RW, -1)>(F, fin, own, m + (int)(~K.bits >> c & 1u), K.bits, rx);
-        }
-    }
     // Explicit sources of the links that the node word cannot express; a warp
     // holds one group.
-    static __device__ __forceinline__ void recorded(R* F, const T* fin, const LbmLinks& L, int n, uint32_t bits,
+    static __device__ __forceinline__ void recorded(R* F, const T* fin, const LbmLinks& L, const NodeLinks& K, int n,
                                                     const LinkRef<R>& rx) {
-        const uint32_t e = __ballot_sync(__activemask(), bits & LBM_LINK_EXC);
-        if (!(bits & LBM_LINK_EXC)) return;
-        const int first = __ldg(L.rec0 + n / LBM_LINK_GROUP);
-        const int32_t* rec = L.rec + (int64_t)LBM_LINK_REC * (first + __popc(e & ((1u << (threadIdx.x & 31)) - 1u)));
+        const int32_t* rec = L.rec;
+        if (!K.record(L, n, rec) || !(K.bits & LBM_LINK_EXC)) return;
 #define LBM_X(S)                                                                              \
     {                                                                                         \
         const int src = __ldg(rec + S);                                                       \
@@ -111,17 +127,10 @@ struct LinkGather {
         const int own = lbm_eoff32(n);
         F[0] = Cd::template dec<0>(fin[own]);
         if constexpr (REF) F[0] = lbm_fma<R>((R)lbm_w(0), rx.at, F[0]);
-        one<1>(F, fin, own, n - 1, K.bits, rx);
-        one<2>(F, fin, own, n + 1, K.bits, rx);
-        row<0>(F, fin, own, K, rx);
-        row<1>(F, fin, own, K, rx);
-        row<2>(F, fin, own, K, rx);
-        row<3>(F, fin, own, K, rx);
-        row<4>(F, fin, own, K, rx);
-        row<5>(F, fin, own, K, rx);
-        row<6>(F, fin, own, K, rx);
-        row<7>(F, fin, own, K, rx);
-        recorded(F, fin, L, n, K.bits, rx);
+#define LBM_G(S) one<S>(F, fin, own, K, n, rx);
+        LBM_ALL_DIRS(LBM_G)
+#undef LBM_G
+        recorded(F, fin, L, K, n, rx);
     }
 };
 

@@ -17,6 +17,7 @@ struct LinkBuild {
     int32_t nx, ny, nz, n_fluid;
     int32_t bc[6];
     int32_t bc_form;
+    int32_t every;        // records on replaced nodes too (two phases: the colours are pulled there)
     uint2* node;
     LbmLinkHead* head;
     int32_t* rec0;
@@ -74,8 +75,9 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
             bits |= LBM_LINK_FACE;
             if (B.bc[f] == LBM_BC_PRESSURE) bits |= LBM_LINK_PRESSURE;
             // (the in-place velocity form reads what was pulled)
-            whole |= B.bc[f] == LBM_BC_PRESSURE || B.bc_form == 0;
+            whole |= !B.every && (B.bc[f] == LBM_BC_PRESSURE || B.bc_form == 0);
         }
+        if (at[0] || at[1] || at[2] || at[3] || at[4] || at[5]) bits |= LBM_LINK_EDGE;
         own = link_row<true>(B, 0, 0, i, j, k);
 #pragma unroll
         for (int d = 0; d < 3; d += 2) {
@@ -155,7 +157,7 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
         const int64_t area[3] = {(int64_t)l.ny * l.nz, (int64_t)l.nx * l.nz, (int64_t)l.nx * l.ny};
         int64_t seam = 0;
         for (int f = 0; f < 6; ++f)
-            if (p.bc[f] == LBM_BC_PERIODIC || (p.bc[f] == LBM_BC_VELOCITY && p.bc_form != 0)) seam += area[f / 2];
+            if (p.two_phase || p.bc[f] == LBM_BC_PERIODIC || (p.bc[f] == LBM_BC_VELOCITY && p.bc_form != 0)) seam += area[f / 2];
         cap += std::min<int64_t>(seam, l.n_fluid) + l.n_fluid / 512;
     }
     for (;;) {
@@ -184,6 +186,7 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
                 B.n_fluid = l.n_fluid;
                 for (int f = 0; f < 6; ++f) B.bc[f] = p.bc[f];
                 B.bc_form = p.bc_form;
+                B.every = p.two_phase;
                 B.node = (uint2*)L.node + l.node_begin;
                 B.head = (LbmLinkHead*)L.head + l.node_begin / LBM_LINK_GROUP;
                 B.rec0 = (int32_t*)L.rec0 + l.node_begin / LBM_LINK_GROUP;

@@ -18,8 +18,8 @@
 // more than 31 from the row's line, has its bit set too, the node's LBM_LINK_EXC
 // bit is set, and an explicit record of 20 int32 holds the source of each such
 // direction (-1 in the others).  Records of 32 nodes are consecutive in node
-// order from rec0.  Nodes whose populations a face condition replaces whole need
-// none for what they pull.
+// order from rec0.  Single-phase nodes whose populations a face condition
+// replaces whole need none for what they pull.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -31,6 +31,7 @@
 #define LBM_LINK_EXC 1u              // the node has a record
 #define LBM_LINK_FACE (1u << 19)     // on a face with a boundary condition
 #define LBM_LINK_PRESSURE (1u << 20) // on a fixed-pressure face
+#define LBM_LINK_EDGE (1u << 21)     // on a face of the lattice
 
 struct __align__(16) LbmLinkHead {
     int32_t start[8];  // rows ordered as lbm_link_ey / lbm_link_ez
@@ -56,6 +57,11 @@ __host__ __device__ constexpr int lbm_link_ey(int r) {
 }
 __host__ __device__ constexpr int lbm_link_ez(int r) {
     return (r == 2 || r == 4 || r == 7) ? 1 : (r == 3 || r == 5 || r == 6) ? -1 : 0;
+}
+__host__ __device__ constexpr int lbm_link_row(int ey, int ez) {
+    for (int r = 0; r < 8; ++r)
+        if (lbm_link_ey(r) == ey && lbm_link_ez(r) == ez) return r;
+    return -1;
 }
 // Direction of row r with e_x = ex (rows 4..7: ex = 0 only).
 __host__ __device__ constexpr int lbm_link_dir(int r, int ex) {

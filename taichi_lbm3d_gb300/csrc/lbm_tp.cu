@@ -19,16 +19,41 @@
 //
 // The colour sums are taken in direction order 0..18, one of the orders the
 // reference's atomic += can produce; the CPU oracle uses the same order, so
-// the two agree bit for bit.  Per node and step the launches move the 152 B of
-// FP32 populations plus rho_r, rho_b, psi, v and the recolouring amounts.
+// the two agree bit for bit.
+//
+// What a node's neighbours pull of it, (rho_r, rho_b, v_x, v_y) as one 16-byte
+// record, v_z and its 9 amounts, launch B leaves behind, so a direction costs three
+// loads.  Sources, and the psi neighbours of launch B away from the lattice
+// faces, come from the neighbour links (lbm_links.cuh).  v and rho are stored
+// only when the caller reads them next (MACROS) or, for v, where a pressure
+// face needs the previous step's.
+//
+// 131^3 drainage, FP32, 894k nodes: 82.7 us a step against 98.4 with six scalar
+// loads a direction and map lookups.  Launch A is bound by L1 wavefronts (every
+// direction reads its own 24 unaligned bytes: 68% of the data pipe), launch B by
+// issue slots and latency at 64 registers.  Storing the 38 recoloured
+// populations instead (two values a direction in launch A) took a third of the
+// wavefronts but 140 MB more DRAM traffic a step: 94 us.
 #include <cuda_runtime.h>
 
-#include <vector>
+#include <algorithm>
 
 #include "lbm_kernels.cuh"
+#include "lbm_linkgather.cuh"
+
+// Resident 128-thread CTAs per SM of the two launches (FP32 and 16-bit), us a step
+// on the same lattice: 10 and 8 82.7; 9 and 7 88.1; 12 and 7 84.2; 11 and 6 86.9.
+#ifndef LBM_TP_MINBLOCKS_A
+#define LBM_TP_MINBLOCKS_A 10
+#endif
+#ifndef LBM_TP_MINBLOCKS_B
+#define LBM_TP_MINBLOCKS_B 8
+#endif
 
 namespace {
 using namespace lbmk;
+
+constexpr int TP_THREADS = 128;
 
 template <typename R>
 struct TpConsts {
@@ -38,6 +63,12 @@ struct TpConsts {
     int32_t psi_bc[6];
     int32_t any_psi_bc;
     R psi_val[6], psi_rr[6], psi_rb[6];
+};
+
+// What launch A pulls of a node, beside v_z and the amounts.
+template <typename R>
+struct __align__(4 * sizeof(R)) ColourRec {
+    R rr, rb, vx, vy;
 };
 
 // Compute_S_local (TP:278-300): s_v and s_other from psi.
@@ -102,28 +133,73 @@ __device__ __forceinline__ void colour_gradient(const TpConsts<R>& T, const int3
     }
 }
 
-// Recolouring amounts of the 9 opposite pairs (TP:346-364): cospsi_p for
-// kk = 2p+1; zero when |C| = 0 (no recolouring).
+// Colour gradient of a node away from the lattice faces: the neighbour at
+// x + e_s is the pull source of the opposite direction.  Same order of terms.
 template <typename R>
-__device__ __forceinline__ void recolour_amounts(R rr, R rb, R vx, R vy, R vz, R Cx, R Cy, R Cz, R cc, R* cs) {
-    const R uv = lbm_usq(vx, vy, vz);
-#define LBM_RC(P)                                                                           \
-    {                                                                                       \
-        constexpr int kk = 2 * P + 1;                                                       \
-        R cp = (R)0;                                                                        \
-        if (cc > (R)0) {                                                                    \
-            const R ga = lbm_feq<kk, R>(rr, vx, vy, vz, uv), gb = lbm_feq<kk + 1, R>(rr, vx, vy, vz, uv); \
-            const R ba = lbm_feq<kk, R>(rb, vx, vy, vz, uv), bb = lbm_feq<kk + 1, R>(rb, vx, vy, vz, uv); \
-            const R ef = lbm_edot<kk, R>(Cx, Cy, Cz);                                       \
-            cp = ga < gb ? ga : gb;                                                         \
-            cp = cp < ba ? cp : ba;                                                         \
-            cp = cp < bb ? cp : bb;                                                         \
-            cp = cp * (ef / cc);                                                            \
-        }                                                                                   \
-        cs[P] = cp;                                                                         \
+__device__ __forceinline__ void colour_gradient_links(const TpConsts<R>& T, const NodeLinks& K, int n, const R* psi,
+                                                      R rr, R rb, R& Cx, R& Cy, R& Cz) {
+    Cx = (R)0;
+    Cy = (R)0;
+    Cz = (R)0;
+#define LBM_CG(S)                                                          \
+    {                                                                      \
+        constexpr int q = lbm_lr(S);                                       \
+        constexpr int ex = lbm_ex(S), ey = lbm_ey(S), ez = lbm_ez(S);      \
+        R ps = T.psi_solid;                                                \
+        if (!(K.bits >> q & 1u)) ps = psi[K.template source<q>(n)];        \
+        const R t = ((R)3.0 * (R)lbm_w(S)) * ps;                           \
+        if constexpr (ex != 0) Cx = ex > 0 ? Cx + t : Cx - t;              \
+        if constexpr (ey != 0) Cy = ey > 0 ? Cy + t : Cy - t;              \
+        if constexpr (ez != 0) Cz = ez > 0 ? Cz + t : Cz - t;              \
     }
-    LBM_RC(0) LBM_RC(1) LBM_RC(2) LBM_RC(3) LBM_RC(4) LBM_RC(5) LBM_RC(6) LBM_RC(7) LBM_RC(8)
+    LBM_ALL_DIRS(LBM_CG)
+#undef LBM_CG
+    R dr = rr - rb;
+    if (dr < (R)0) dr = -dr;
+    if (dr > (R)0.9 && (K.bits & 0x7fffeu)) {
+        Cx = (R)0;
+        Cy = (R)0;
+        Cz = (R)0;
+    }
+}
+
+// Normal C / |C| and recolouring amounts of the 9 opposite pairs (TP:346-364):
+// cospsi_p for kk = 2p+1; all zero when |C| = 0 (no recolouring).
+template <typename R>
+__device__ __forceinline__ void recolour_amounts(R rr, R rb, R vx, R vy, R vz, R Cx, R Cy, R Cz, R cc, R u15, R* nrm,
+                                                 R* cs) {
+    R q[12];
+#pragma unroll
+    for (int p = 0; p < 12; ++p) q[p] = (R)0;
+    if (cc > (R)0) {
+        q[9] = Cx;
+        q[10] = Cy;
+        q[11] = Cz;
+#define LBM_RC(P) q[P] = lbm_edot<2 * P + 1, R>(Cx, Cy, Cz);
+        LBM_RC(0) LBM_RC(1) LBM_RC(2) LBM_RC(3) LBM_RC(4) LBM_RC(5) LBM_RC(6) LBM_RC(7) LBM_RC(8)
 #undef LBM_RC
+        quotients(q, cc);
+#define LBM_RC(P)                                                                                       \
+    {                                                                                                   \
+        constexpr int kk = 2 * P + 1;                                                                   \
+        /* feq of kk and kk + 1 (e.u and -e.u) for both colours (lbm_feq, term by term) */              \
+        const R eu = lbm_edot<kk, R>(vx, vy, vz);                                                       \
+        const R e3 = (R)3.0 * eu, e45 = ((R)4.5 * eu) * eu;                                             \
+        const R tp = (((R)1.0 + e3) + e45) - u15, tm = (((R)1.0 - e3) + e45) - u15;                     \
+        const R wr = (R)lbm_w(kk) * rr, wb = (R)lbm_w(kk) * rb;                                         \
+        const R ga = wr * tp, gb = wr * tm, ba = wb * tp, bb = wb * tm;                                 \
+        R cp = ga < gb ? ga : gb;                                                                       \
+        cp = cp < ba ? cp : ba;                                                                         \
+        cp = cp < bb ? cp : bb;                                                                         \
+        q[P] = cp * q[P];                                                                               \
+    }
+        LBM_RC(0) LBM_RC(1) LBM_RC(2) LBM_RC(3) LBM_RC(4) LBM_RC(5) LBM_RC(6) LBM_RC(7) LBM_RC(8)
+#undef LBM_RC
+    }
+#pragma unroll
+    for (int p = 0; p < 9; ++p) cs[p] = q[p];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) nrm[d] = q[9 + d];
 }
 
 // Two-phase MRT collision (TP:302-344) of F in place.
@@ -188,37 +264,36 @@ __device__ __forceinline__ void collide_tp(R* F, R r, R vx, R vy, R vz, R cc, R 
     else mrt_back<R>(m, F);
 }
 
-// Everything B does after the macros: colour gradient, collision, recolouring.
+// Everything B does after the macros: recolouring amounts, collision, and what
+// the next launch A pulls.
 template <int STORE, bool FORCE>
 __device__ __forceinline__ void tp_collide_and_store(typename Codec<STORE>::R* F, typename Codec<STORE>::R r,
                                                      typename Codec<STORE>::R vx, typename Codec<STORE>::R vy,
-                                                     typename Codec<STORE>::R vz, int n, int i, int j, int k,
+                                                     typename Codec<STORE>::R vz, int n,
+                                                     typename Codec<STORE>::R ref_own,
                                                      const TpConsts<typename Codec<STORE>::R>& T,
-                                                     const int32_t* __restrict__ map,
-                                                     const typename Codec<STORE>::R* __restrict__ psi,
+                                                     typename Codec<STORE>::R Cx, typename Codec<STORE>::R Cy,
+                                                     typename Codec<STORE>::R Cz, typename Codec<STORE>::R psi,
                                                      typename Codec<STORE>::R rr, typename Codec<STORE>::R rb,
                                                      typename Codec<STORE>::T* __restrict__ fout,
+                                                     ColourRec<typename Codec<STORE>::R>* __restrict__ crec,
+                                                     typename Codec<STORE>::R* __restrict__ pull_vz,
                                                      typename Codec<STORE>::R* __restrict__ cs_out) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
-    R Cx, Cy, Cz;
-    colour_gradient<R>(T, map, psi, i, j, k, rr, rb, Cx, Cy, Cz);
-    const R cc = sqrt(lbm_usq(Cx, Cy, Cz));
-    R n0 = (R)0, n1 = (R)0, n2 = (R)0;
-    if (cc > (R)0) {
-        n0 = Cx / cc;
-        n1 = Cy / cc;
-        n2 = Cz / cc;
-    }
-    R sv, so;
-    s_local<R>(T, psi[n], sv, so);
-    collide_tp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, cc, n0, n1, n2, sv, so, T);
-    store_node<STORE>(F, fout, n, lbm_ref_at(sp_ref(T.sp), i), T.sp.seed);
-    R cs[9];
-    recolour_amounts<R>(rr, rb, vx, vy, vz, Cx, Cy, Cz, cc, cs);
     const int64_t np = T.sp.np;
+    const R cc = sqrt(lbm_usq(Cx, Cy, Cz));
+    const R u15 = (R)1.5 * lbm_usq(vx, vy, vz);
+    R nrm[3], cs[9];
+    recolour_amounts<R>(rr, rb, vx, vy, vz, Cx, Cy, Cz, cc, u15, nrm, cs);
 #pragma unroll
     for (int p = 0; p < 9; ++p) cs_out[p * np + n] = cs[p];
+    crec[n] = {rr, rb, vx, vy};
+    pull_vz[n] = vz;
+    R sv, so;
+    s_local<R>(T, psi, sv, so);
+    collide_tp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, cc, nrm[0], nrm[1], nrm[2], sv, so, T);
+    store_node<STORE>(F, fout, n, ref_own, T.sp.seed);
 }
 
 // Programmatic dependent launch between the step's launches (A, B, next A):
@@ -228,7 +303,6 @@ __device__ __forceinline__ void tp_collide_and_store(typename Codec<STORE>::R* F
 __device__ __forceinline__ void tp_pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-__device__ __forceinline__ void tp_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename K, typename... Args>
 cudaError_t tp_launch_pdl(K kernel, int grid, int block, cudaStream_t stream, Args... args) {
@@ -245,76 +319,82 @@ cudaError_t tp_launch_pdl(K kernel, int grid, int block, cudaStream_t stream, Ar
 }
 
 // ---------------------------------------------------------------- launch A
-template <int Q, typename R>
-__device__ __forceinline__ void colour_pull_one(const TpConsts<R>& T, const int32_t* __restrict__ map,
-                                                const Rows& rows, int n, int i, int xm, int xp, bool xwrap,
-                                                const R* __restrict__ rr, const R* __restrict__ rb,
-                                                const R* __restrict__ v, const R* __restrict__ cs, R& acc_r,
-                                                R& acc_b) {
-    const int64_t np = T.sp.np;
-    int src = n;
+// Direction Q: what the node at x - e_Q (or, bounced, the node itself in the
+// opposite direction) sends.  EXC: some node of the warp has a record.
+template <int Q, bool EXC, typename R>
+__device__ __forceinline__ void colour_pull_one(const NodeLinks& K, const int32_t* rec, int64_t np, int n,
+                                                const ColourRec<R>* crec, const R* pull_vz, const R* cs,
+                                                R& acc_r, R& acc_b) {
+    bool bounce = false;
+    int m = n;
     if constexpr (Q != 0) {
-        constexpr int ex = lbm_ex(Q), ey = lbm_ey(Q), ez = lbm_ez(Q);
-        const int row = rows.r[1 - ey][1 - ez];
-        const int x = ex > 0 ? xm : (ex < 0 ? xp : i);
-        src = xwrap ? __ldg(map + (row - i + x)) : __ldg(map + row - ex);
+        bounce = K.bits >> Q & 1u;
+        if (!bounce) m = K.template source<Q>(n);
+        if constexpr (EXC)
+            if (bounce && (K.bits & LBM_LINK_EXC)) {
+                const int to = __ldg(rec + Q);
+                if (to >= 0) {
+                    m = to;
+                    bounce = false;
+                }
+            }
     }
-    const bool bounce = src < 0;
-    const int m = bounce ? n : src;
-    const R vx = v[m], vy = v[np + m], vz = v[2 * np + m];
-    const R uv = lbm_usq(vx, vy, vz);
-    R eu = lbm_edot<Q, R>(vx, vy, vz);
+    const ColourRec<R> a = crec[m];
+    const R vz = pull_vz[m];
+    R eu = lbm_edot<Q, R>(a.vx, a.vy, vz);
     if (bounce) eu = -eu;  // direction LR[Q] at the node itself: e_LR = -e_Q
     R t = (R)1.0 + (R)3.0 * eu;
     t = t + ((R)4.5 * eu) * eu;
-    t = t - (R)1.5 * uv;
-    R gr = ((R)lbm_w(Q) * rr[m]) * t;
-    R gb = ((R)lbm_w(Q) * rb[m]) * t;
+    t = t - (R)1.5 * lbm_usq(a.vx, a.vy, vz);
+    R gr = ((R)lbm_w(Q) * a.rr) * t;
+    R gb = ((R)lbm_w(Q) * a.rb) * t;
     if constexpr (Q != 0) {
         // pair kk = 2p+1 gets +cospsi for red (kk) and -cospsi (kk+1); blue opposite
-        const R c = cs[((Q - 1) >> 1) * np + m];
-        const bool plus = ((Q & 1) != 0) != bounce;
-        gr = plus ? gr + c : gr - c;
-        gb = plus ? gb - c : gb + c;
+        R c = cs[((Q - 1) >> 1) * np + m];
+        if (((Q & 1) != 0) == bounce) c = -c;
+        gr = gr + c;
+        gb = gb - c;
     }
     acc_r = acc_r + gr;
     acc_b = acc_b + gb;
 }
 
-// 4 CTAs of 256 per SM (64 registers): the 19 source gathers of 6 values each
-// stay in flight together; at the compiler's own 40 registers (6 CTAs) the
-// 131^3 drainage step runs 4.7% slower, at 80 registers (3 CTAs) 23% slower.
 template <typename R>
-__global__ void __launch_bounds__(256, 4) tp_colour_kernel(const __grid_constant__ TpConsts<R> T,
-                                                        const R* __restrict__ rr_in, const R* __restrict__ rb_in,
-                                                        const R* __restrict__ v, const R* __restrict__ cs,
-                                                        R* __restrict__ rr_out, R* __restrict__ rb_out,
-                                                        R* __restrict__ psi_out, const int32_t* __restrict__ map,
-                                                        const uint32_t* __restrict__ coord) {
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : LBM_TP_MINBLOCKS_A) tp_colour_kernel(
+    const __grid_constant__ TpConsts<R> T, const ColourRec<R>* crec_prev, const R* vz_prev, const R* cs_prev,
+    R* __restrict__ rr_out, R* __restrict__ rb_out, R* __restrict__ psi_out, const __grid_constant__ LbmLinks L,
+    const uint32_t* __restrict__ coord) {
     tp_pdl_launch_dependents();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= T.sp.n_fluid) return;
-    const uint32_t pc = __ldg(coord + n);
-    const int i = lbm_pi(pc), j = lbm_pj(pc), k = lbm_pk(pc);
-    const int nx = T.sp.nx, ny = T.sp.ny, nz = T.sp.nz;
-    const int xm = i == 0 ? nx - 1 : i - 1, xp = i == nx - 1 ? 0 : i + 1;
-    const int ym = j == 0 ? ny - 1 : j - 1, yp = j == ny - 1 ? 0 : j + 1;
-    const int zm = k == 0 ? nz - 1 : k - 1, zp = k == nz - 1 ? 0 : k + 1;
-    const Rows rows = make_rows(nx, ny, i, j, k, ym, yp, zm, zp);
-    const bool xwrap = !(i > 0 && i < nx - 1);
-    tp_pdl_wait();  // v, cs of the previous flow launch; psi is rewritten below
+    NodeLinks K;
+    K.load(L, n);
+    const int32_t* rec = L.rec;
+    const bool exc = K.record(L, n, rec);
+    // records and amounts of the previous flow launch; psi is rewritten below
+    const ColourRec<R>* crec = wait_previous(crec_prev);
+    const R* vz = launder(vz_prev);
+    const R* cs = launder(cs_prev);
     R ar = (R)0, ab = (R)0;
-#define LBM_CP(Q) colour_pull_one<Q, R>(T, map, rows, n, i, xm, xp, xwrap, rr_in, rb_in, v, cs, ar, ab);
-    LBM_CP(0) LBM_ALL_DIRS(LBM_CP)
+    if (exc) {
+#define LBM_CP(Q) colour_pull_one<Q, true, R>(K, rec, T.sp.np, n, crec, vz, cs, ar, ab);
+        LBM_CP(0) LBM_ALL_DIRS(LBM_CP)
 #undef LBM_CP
+    } else {
+#define LBM_CP(Q) colour_pull_one<Q, false, R>(K, rec, T.sp.np, n, crec, vz, cs, ar, ab);
+        LBM_CP(0) LBM_ALL_DIRS(LBM_CP)
+#undef LBM_CP
+    }
     R psi = ar - ab / (ar + ab);  // TP:606 as written
-    if (T.any_psi_bc) {
+    if (T.any_psi_bc && (K.bits & LBM_LINK_EDGE)) {
+        const uint32_t pc = __ldg(coord + n);
+        const int i = lbm_pi(pc), j = lbm_pj(pc), k = lbm_pk(pc);
 #pragma unroll 1
         for (int f = 0; f < 6; ++f) {
             if (!T.psi_bc[f]) continue;
             const int hi = f & 1;
             const int c = f < 2 ? i : (f < 4 ? j : k);
-            const int nmax = f < 2 ? nx : (f < 4 ? ny : nz);
+            const int nmax = f < 2 ? T.sp.nx : (f < 4 ? T.sp.ny : T.sp.nz);
             if (c != (hi ? nmax - 1 : 0)) continue;
             psi = T.psi_val[f];
             ar = T.psi_rr[f];
@@ -327,67 +407,87 @@ __global__ void __launch_bounds__(256, 4) tp_colour_kernel(const __grid_constant
 }
 
 // ---------------------------------------------------------------- launch B
-template <int STORE, bool FORCE>
-__global__ void __launch_bounds__(256) tp_flow_kernel(const __grid_constant__ TpConsts<typename Codec<STORE>::R> T,
-                                                      const typename Codec<STORE>::T* __restrict__ fin,
-                                                      typename Codec<STORE>::T* __restrict__ fout,
-                                                      const int32_t* __restrict__ map,
-                                                      const uint32_t* __restrict__ coord,
-                                                      typename Codec<STORE>::R* __restrict__ v,
-                                                      typename Codec<STORE>::R* __restrict__ rho_out,
-                                                      const typename Codec<STORE>::R* __restrict__ rr,
-                                                      const typename Codec<STORE>::R* __restrict__ rb,
-                                                      const typename Codec<STORE>::R* __restrict__ psi,
-                                                      typename Codec<STORE>::R* __restrict__ cs_out) {
+template <int STORE, bool FORCE, bool MACROS>
+__global__ void __launch_bounds__(128, STORE == LBM_STORE_F64 ? 2 : LBM_TP_MINBLOCKS_B) tp_flow_kernel(
+    const __grid_constant__ TpConsts<typename Codec<STORE>::R> T, const typename Codec<STORE>::T* f_prev,
+    typename Codec<STORE>::T* __restrict__ fout, const int32_t* __restrict__ map, const uint32_t* __restrict__ coord,
+    const __grid_constant__ LbmLinks L, typename Codec<STORE>::R* v, typename Codec<STORE>::R* __restrict__ rho_out,
+    const typename Codec<STORE>::R* rr_new, const typename Codec<STORE>::R* rb_new,
+    const typename Codec<STORE>::R* psi_new, ColourRec<typename Codec<STORE>::R>* __restrict__ crec,
+    typename Codec<STORE>::R* __restrict__ pull_vz, typename Codec<STORE>::R* __restrict__ cs_out) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
     const SpConsts<R>& C = T.sp;
     tp_pdl_launch_dependents();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= C.n_fluid) return;
-    const uint32_t pc = __ldg(coord + n);
-    const int i = lbm_pi(pc), j = lbm_pj(pc), k = lbm_pk(pc);
+    NodeLinks K;
+    K.load(L, n);
+    int i = 0, j = 0, k = 0;
+    if (Cd::RHOREF || (K.bits & (LBM_LINK_EDGE | LBM_LINK_EXC))) {
+        const uint32_t pc = __ldg(coord + n);
+        i = lbm_pi(pc);
+        j = lbm_pj(pc);
+        k = lbm_pk(pc);
+    }
+    const LinkRef<R> rx(sp_ref(C), i, C.nx);
     const int64_t np = C.np;
-    tp_pdl_wait();  // rho_r, rho_b, psi of the colour launch; f, v, cs of the previous step
+    // rho_r, rho_b, psi of the colour launch; f, v of the previous step
+    const auto* fin = wait_previous(f_prev);
+    const R* psi = launder(psi_new);
+    const R rr = launder(rr_new)[n], rb = launder(rb_new)[n];
     R F[19];
-    gather_node<STORE>(F, fin, map, n, C.nx, C.ny, C.nz, i, j, k, sp_ref(C));
-    if (C.any_bc && on_face(i, j, k, C, false)) apply_faces<R, Cd::DEV>(F, i, j, k, n, C, map, v);  // v: previous step
+    LinkGather<STORE, Cd::RHOREF>::all(F, fin, L, K, n, rx);
+    if (K.bits & LBM_LINK_FACE) apply_faces<R, Cd::DEV>(F, i, j, k, n, C, map, v);  // v: previous step
     R r = F[0];
 #pragma unroll
     for (int s = 1; s < 19; ++s) r = r + F[s];
     const R rho = Cd::DEV ? (R)1 + r : r;
     R vx = vsum<0>(F), vy = vsum<1>(F), vz = vsum<2>(F);
-    vx = vx / rho;
-    vy = vy / rho;
-    vz = vz / rho;
-    if constexpr (FORCE) {
-        vx = vx + C.fhalf[0] / rho;
-        vy = vy + C.fhalf[1] / rho;
-        vz = vz + C.fhalf[2] / rho;
+    velocity<R, FORCE>(vx, vy, vz, rho, C);
+    if (MACROS) rho_out[n] = rho;
+    if (MACROS || (K.bits & LBM_LINK_PRESSURE)) {
+        v[n] = vx;
+        v[np + n] = vy;
+        v[2 * np + n] = vz;
     }
-    rho_out[n] = rho;
-    v[n] = vx;
-    v[np + n] = vy;
-    v[2 * np + n] = vz;
-    tp_collide_and_store<STORE, FORCE>(F, r, vx, vy, vz, n, i, j, k, T, map, psi, rr[n], rb[n], fout, cs_out);
+    R Cx, Cy, Cz;
+    if (K.bits & (LBM_LINK_EDGE | LBM_LINK_EXC)) colour_gradient<R>(T, map, psi, i, j, k, rr, rb, Cx, Cy, Cz);
+    else colour_gradient_links<R>(T, K, n, psi, rr, rb, Cx, Cy, Cz);
+    tp_collide_and_store<STORE, FORCE>(F, r, vx, vy, vz, n, rx.at, T, Cx, Cy, Cz, psi[n], rr, rb, fout, crec,
+                                       pull_vz, cs_out);
 }
 
 // Initial state (TP:174-187) and the first collision: rho = 1, v = 0, F = feq(1, 0),
-// rho_r = (psi + 1)/2, rho_b = 1 - rho_r, psi = the input psi.
+// rho_r = (psi + 1)/2, rho_b = 1 - rho_r, psi = the input psi (dense, psi0).
+template <int STORE>
+__global__ void tp_psi_kernel(const __grid_constant__ TpConsts<typename Codec<STORE>::R> T,
+                              const uint32_t* __restrict__ coord, const float* __restrict__ psi0,
+                              typename Codec<STORE>::R* __restrict__ psi) {
+    const int n = blockIdx.x * blockDim.x + threadIdx.x;
+    if (n >= T.sp.n_fluid) return;
+    const uint32_t pc = __ldg(coord + n);
+    psi[n] = (typename Codec<STORE>::R)psi0[lbm_pi(pc) + (int64_t)T.sp.nx * (lbm_pj(pc) + (int64_t)T.sp.ny * lbm_pk(pc))];
+}
+
 template <int STORE, bool FORCE>
 __global__ void tp_init_kernel(const __grid_constant__ TpConsts<typename Codec<STORE>::R> T,
                                typename Codec<STORE>::T* __restrict__ fout, const int32_t* __restrict__ map,
                                const uint32_t* __restrict__ coord, typename Codec<STORE>::R* __restrict__ v,
                                typename Codec<STORE>::R* __restrict__ rho_out, typename Codec<STORE>::R* __restrict__ rr,
                                typename Codec<STORE>::R* __restrict__ rb, const typename Codec<STORE>::R* __restrict__ psi,
+                               ColourRec<typename Codec<STORE>::R>* __restrict__ crec,
+                               typename Codec<STORE>::R* __restrict__ pull_vz,
                                typename Codec<STORE>::R* __restrict__ cs_out) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= T.sp.n_fluid) return;
     const uint32_t pc = __ldg(coord + n);
+    const int i = lbm_pi(pc), j = lbm_pj(pc), k = lbm_pk(pc);
     const int64_t np = T.sp.np;
-    const R r0 = (psi[n] + (R)1.0) / (R)2.0;
+    const R p = psi[n];
+    const R r0 = (p + (R)1.0) / (R)2.0;
     const R b0 = (R)1.0 - r0;
     rr[n] = r0;
     rb[n] = b0;
@@ -398,8 +498,10 @@ __global__ void tp_init_kernel(const __grid_constant__ TpConsts<typename Codec<S
     R F[19];
     if constexpr (Cd::DEV) lbm_feq_dev_all<R>((R)0, (R)0, (R)0, (R)0, F);
     else lbm_feq_all<R>((R)1.0, (R)0, (R)0, (R)0, F);
-    tp_collide_and_store<STORE, FORCE>(F, Cd::DEV ? (R)0 : (R)1.0, (R)0, (R)0, (R)0, n, lbm_pi(pc), lbm_pj(pc),
-                                       lbm_pk(pc), T, map, psi, r0, b0, fout, cs_out);
+    R Cx, Cy, Cz;
+    colour_gradient<R>(T, map, psi, i, j, k, r0, b0, Cx, Cy, Cz);
+    tp_collide_and_store<STORE, FORCE>(F, Cd::DEV ? (R)0 : (R)1.0, (R)0, (R)0, (R)0, n, lbm_ref_at(sp_ref(T.sp), i), T,
+                                       Cx, Cy, Cz, p, r0, b0, fout, crec, pull_vz, cs_out);
 }
 
 template <typename R>
@@ -432,45 +534,37 @@ int tp_init_t(LbmHandle* h) {
     using R = typename Codec<STORE>::R;
     using Tt = typename Codec<STORE>::T;
     const TpConsts<R> T = make_tp<R>(h);
-    // psi of the fluid nodes, in node order
-    int rc = geom_host_index(h);
-    if (rc) return rc;
-    std::vector<R> hp(h->np, (R)0);
-    for (int32_t n = 0; n < h->n_fluid; ++n) hp[n] = (R)h->psi0[h->cell_of_node[n]];
-    rc = lbm_cuda_check(h, cudaMemcpyAsync(h->d_psi, hp.data(), sizeof(R) * h->np, cudaMemcpyHostToDevice, h->stream),
-                            "copy psi");
-    if (rc) return rc;
     h->cur = 0;
-    h->ccur = 0;
     const int grid = (int)((h->n_fluid + h->block - 1) / h->block);
+    tp_psi_kernel<STORE><<<grid, h->block, 0, h->stream>>>(T, h->d_coord, h->d_psi0, (R*)h->d_psi);
     auto k = h->force ? tp_init_kernel<STORE, true> : tp_init_kernel<STORE, false>;
     k<<<grid, h->block, 0, h->stream>>>(T, (Tt*)h->d_f[0], h->d_map, h->d_coord, (R*)h->d_v, (R*)h->d_rho,
-                                        (R*)h->d_rr[0], (R*)h->d_rb[0], (const R*)h->d_psi, (R*)h->d_cs);
-    rc = lbm_cuda_check(h, cudaGetLastError(), "tp_init_kernel launch");
+                                        (R*)h->d_rr, (R*)h->d_rb, (const R*)h->d_psi, (ColourRec<R>*)h->d_crec,
+                                        (R*)h->d_pull_vz, (R*)h->d_cs);
+    int rc = lbm_cuda_check(h, cudaGetLastError(), "tp_init_kernel launch");
     if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "tp_init");
     return rc;
 }
 
-template <int STORE>
-int tp_steps_t(LbmHandle* h, int32_t nsteps) {
+template <int STORE, bool FORCE>
+int tp_steps_t(LbmHandle* h, int32_t nsteps, bool macros_last) {
     using R = typename Codec<STORE>::R;
     using Tt = typename Codec<STORE>::T;
     TpConsts<R> T = make_tp<R>(h);
-    const int grid = (int)((h->n_fluid + h->block - 1) / h->block);
-    auto kb = h->force ? tp_flow_kernel<STORE, true> : tp_flow_kernel<STORE, false>;
+    const int block = std::min<int>(h->block, TP_THREADS);
+    const int grid = (int)((h->n_fluid + block - 1) / block);
     for (int32_t it = 0; it < nsteps; ++it) {
         T.sp.seed = (uint32_t)(h->steps_done + it);   // global step index: rounding bits of this step
-        const int c = h->ccur;
-        cudaError_t e = tp_launch_pdl(tp_colour_kernel<R>, grid, h->block, h->stream, T, (const R*)h->d_rr[c],
-                                      (const R*)h->d_rb[c], (const R*)h->d_v, (const R*)h->d_cs, (R*)h->d_rr[c ^ 1],
-                                      (R*)h->d_rb[c ^ 1], (R*)h->d_psi, (const int32_t*)h->d_map,
-                                      (const uint32_t*)h->d_coord);
+        cudaError_t e = tp_launch_pdl(tp_colour_kernel<R>, grid, block, h->stream, T, (const ColourRec<R>*)h->d_crec,
+                                      (const R*)h->d_pull_vz, (const R*)h->d_cs, (R*)h->d_rr, (R*)h->d_rb,
+                                      (R*)h->d_psi, h->links, (const uint32_t*)h->d_coord);
         int rc = lbm_cuda_check(h, e != cudaSuccess ? e : cudaGetLastError(), "tp_colour_kernel launch");
         if (rc) return rc;
-        h->ccur ^= 1;
-        e = tp_launch_pdl(kb, grid, h->block, h->stream, T, (const Tt*)h->d_f[h->cur], (Tt*)h->d_f[h->cur ^ 1],
-                          (const int32_t*)h->d_map, (const uint32_t*)h->d_coord, (R*)h->d_v, (R*)h->d_rho,
-                          (const R*)h->d_rr[h->ccur], (const R*)h->d_rb[h->ccur], (const R*)h->d_psi, (R*)h->d_cs);
+        auto kb = macros_last && it == nsteps - 1 ? tp_flow_kernel<STORE, FORCE, true> : tp_flow_kernel<STORE, FORCE, false>;
+        e = tp_launch_pdl(kb, grid, block, h->stream, T, (const Tt*)h->d_f[h->cur], (Tt*)h->d_f[h->cur ^ 1],
+                          (const int32_t*)h->d_map, (const uint32_t*)h->d_coord, h->links, (R*)h->d_v, (R*)h->d_rho,
+                          (const R*)h->d_rr, (const R*)h->d_rb, (const R*)h->d_psi, (ColourRec<R>*)h->d_crec,
+                          (R*)h->d_pull_vz, (R*)h->d_cs);
         rc = lbm_cuda_check(h, e != cudaSuccess ? e : cudaGetLastError(), "tp_flow_kernel launch");
         if (rc) return rc;
         h->cur ^= 1;
@@ -478,12 +572,16 @@ int tp_steps_t(LbmHandle* h, int32_t nsteps) {
     return LBM_OK;
 }
 
+template <int STORE>
+int tp_steps(LbmHandle* h, int32_t n, bool macros_last) {
+    return h->force ? tp_steps_t<STORE, true>(h, n, macros_last) : tp_steps_t<STORE, false>(h, n, macros_last);
+}
+
 }  // namespace
 
 int tp_launch_init(LbmHandle* h) {
     if (h->n_fluid == 0) {   // all solid: nothing to initialise (an empty grid is not launchable)
         h->cur = 0;
-        h->ccur = 0;
         return LBM_OK;
     }
     switch (h->p.storage) {
@@ -496,14 +594,14 @@ int tp_launch_init(LbmHandle* h) {
     return lbm_set_err(h, LBM_EINVAL, "unknown storage");
 }
 
-int tp_launch_steps(LbmHandle* h, int32_t n, bool) {
+int tp_launch_steps(LbmHandle* h, int32_t n, bool macros_last) {
     if (h->n_fluid == 0) return LBM_OK;
     switch (h->p.storage) {
-    case LBM_STORE_F32: return tp_steps_t<LBM_STORE_F32>(h, n);
-    case LBM_STORE_F16_DEV: return tp_steps_t<LBM_STORE_F16_DEV>(h, n);
-    case LBM_STORE_BF16_DEV: return tp_steps_t<LBM_STORE_BF16_DEV>(h, n);
-    case LBM_STORE_F32_DEV: return tp_steps_t<LBM_STORE_F32_DEV>(h, n);
-    case LBM_STORE_F64: return tp_steps_t<LBM_STORE_F64>(h, n);
+    case LBM_STORE_F32: return tp_steps<LBM_STORE_F32>(h, n, macros_last);
+    case LBM_STORE_F16_DEV: return tp_steps<LBM_STORE_F16_DEV>(h, n, macros_last);
+    case LBM_STORE_BF16_DEV: return tp_steps<LBM_STORE_BF16_DEV>(h, n, macros_last);
+    case LBM_STORE_F32_DEV: return tp_steps<LBM_STORE_F32_DEV>(h, n, macros_last);
+    case LBM_STORE_F64: return tp_steps<LBM_STORE_F64>(h, n, macros_last);
     }
     return lbm_set_err(h, LBM_EINVAL, "unknown storage");
 }

@@ -72,7 +72,7 @@ using namespace lbmk;
 // 38.0k / 32.0k, FP32 deviation form 36.3k / 30.9k, FP32 23.5k / 20.2k.  Bound by
 // issue slots as the single-lattice kernel.  Tiles of 64 and 128 threads run
 // alike (38.1k, 38.0k FP16), of 256 36.0k.
-template <int STORE, bool FORCE, bool CHECK>
+template <int STORE, int FORCE, bool CHECK>
 __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Codec<STORE>::DEV ? 4 : 5)
     batch_step_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C, const BatchTile* __restrict__ tiles,
                       const typename Codec<STORE>::T* f_prev, typename Codec<STORE>::T* __restrict__ fout,
@@ -104,12 +104,8 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Co
 #pragma unroll
         for (int s = 1; s < 19; ++s) r = r + F[s];
         const R rho = Cd::DEV ? (R)1 + r : r;
-        R vx = vsum<0>(F) / rho, vy = vsum<1>(F) / rho, vz = vsum<2>(F) / rho;
-        if constexpr (FORCE) {
-            vx = vx + C.fhalf[0] / rho;
-            vy = vy + C.fhalf[1] / rho;
-            vz = vz + C.fhalf[2] / rho;
-        }
+        R vx = vsum<0>(F), vy = vsum<1>(F), vz = vsum<2>(F);
+        velocity<R, FORCE>(vx, vy, vz, rho, C.fhalf);
         if constexpr (CHECK) acc += (double)vx;
         collide_sp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, C);
         store_node<STORE>(F, out, n, (R)0, seed);
@@ -202,12 +198,19 @@ int launch_one(LbmBatch* b, int k, bool check, cudaStream_t s) {
         e = cudaLaunchKernelEx(&cfg, kern, C, (const BatchTile*)b->d_tiles, fin, fout, h->links,
                                (const uint32_t*)b->d_seed, b->d_partial);
     };
-    if (h->force) {
-        if (check) args(batch_step_kernel<STORE, true, true>);
-        else args(batch_step_kernel<STORE, true, false>);
-    } else {
-        if (check) args(batch_step_kernel<STORE, false, true>);
-        else args(batch_step_kernel<STORE, false, false>);
+    constexpr int X = Cd::DEV ? FORCE_ANY : FORCE_X;   // (the deviation form has one kernel for every force)
+    switch (force_kind(h)) {
+    case FORCE_NONE:
+        if (check) args(batch_step_kernel<STORE, FORCE_NONE, true>);
+        else args(batch_step_kernel<STORE, FORCE_NONE, false>);
+        break;
+    case FORCE_X:
+        if (check) args(batch_step_kernel<STORE, X, true>);
+        else args(batch_step_kernel<STORE, X, false>);
+        break;
+    default:
+        if (check) args(batch_step_kernel<STORE, FORCE_ANY, true>);
+        else args(batch_step_kernel<STORE, FORCE_ANY, false>);
     }
     return lbm_cuda_check(h, e != cudaSuccess ? e : cudaGetLastError(), "batch_step_kernel launch");
 }

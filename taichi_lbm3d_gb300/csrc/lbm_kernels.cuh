@@ -272,21 +272,82 @@ __device__ __forceinline__ void quotients(double (&a)[K], double b) {
     for (int k = 0; k < K; ++k) a[k] = a[k] / b;
 }
 
+// a / N for the constant divisors of the class Guo term: the same correction with
+// the reciprocal rounded to nearest; equal to the division for every FP32
+// significand (tests/test_quotients.py goes through all of them).
+template <int N>
+__device__ __forceinline__ float div_const(float a) {
+    const float q = a * (float)(1.0 / N);
+    return lbm_fma<float>(lbm_fma<float>(q, -(float)N, a), (float)(1.0 / N), q);
+}
+template <int N>
+__device__ __forceinline__ double div_const(double a) {
+    return a / (double)N;
+}
+
+// Body force of a kernel: none, any, or along x only (the common case, which
+// spares the dense Guo term its zero products).
+enum { FORCE_NONE = 0, FORCE_ANY = 1, FORCE_X = 2 };
+
+inline int force_kind(const LbmHandle* h) {
+    if (!h->force) return FORCE_NONE;
+    return h->p.force[1] == 0.0 && h->p.force[2] == 0.0 ? FORCE_X : FORCE_ANY;
+}
+
 // v = j / rho, plus half the body force over rho (SP:382-388).
-template <typename R, bool FORCE>
-__device__ __forceinline__ void velocity(R& vx, R& vy, R& vz, R rho, const SpConsts<R>& C) {
-    if constexpr (FORCE) {
-        R q[6] = {vx, vy, vz, C.fhalf[0], C.fhalf[1], C.fhalf[2]};
+template <typename R, int FORCE>
+__device__ __forceinline__ void velocity(R& vx, R& vy, R& vz, R rho, const R (&fhalf)[3]) {
+    if constexpr (FORCE == FORCE_ANY) {
+        R q[6] = {vx, vy, vz, fhalf[0], fhalf[1], fhalf[2]};
         quotients(q, rho);
         vx = q[0] + q[3];
         vy = q[1] + q[4];
         vz = q[2] + q[5];
     } else {
-        R q[3] = {vx, vy, vz};
+        R q[4] = {vx, vy, vz, fhalf[0]};
+        if constexpr (FORCE == FORCE_NONE) q[3] = (R)0;
         quotients(q, rho);
-        vx = q[0];
+        vx = FORCE == FORCE_X ? q[0] + q[3] : q[0];
         vy = q[1];
         vz = q[2];
+    }
+}
+
+// w_l times the Guo term of each direction (dense form), convention as in
+// SpConsts::guo: class (/3, /9, SP:236), scripts (TP:246), standard (3, 9; c_s^2 = 1/3).
+template <typename R, int FORCE>
+__device__ __forceinline__ void guo_dense(R* G, R vx, R vy, R vz, const R (&fext)[3], int guo) {
+    const R fx = fext[0], fy = fext[1], fz = fext[2];
+    auto conv = [&](R a, R ee) {
+        if (guo == 0) return div_const<3>(a) + div_const<9>(ee);
+        if (guo == 1) return a + ee;
+        return (R)3.0 * a + (R)9.0 * ee;
+    };
+    if constexpr (FORCE == FORCE_X) {
+        // (e_x - v_x) F_x is all that is left of (e - v).F, e_x F_x of e.F: the
+        // general form adds products with zeros to them
+        const R am = ((R)-1 - vx) * fx, a0 = ((R)0 - vx) * fx, ap = ((R)1 - vx) * fx;
+        const R g0 = conv(a0, (R)0);
+#define LBM_GX(S)                                                                     \
+    if constexpr (lbm_ex(S) == 0) G[S] = (R)lbm_w(S) * g0;                            \
+    else {                                                                            \
+        const R ee = lbm_edot<S, R>(vx, vy, vz) * fx;                                 \
+        G[S] = (R)lbm_w(S) * (lbm_ex(S) > 0 ? conv(ap, ee) : conv(am, -ee));          \
+    }
+        LBM_GX(0) LBM_GX(1) LBM_GX(2) LBM_GX(3) LBM_GX(4) LBM_GX(5) LBM_GX(6) LBM_GX(7) LBM_GX(8) LBM_GX(9)
+        LBM_GX(10) LBM_GX(11) LBM_GX(12) LBM_GX(13) LBM_GX(14) LBM_GX(15) LBM_GX(16) LBM_GX(17) LBM_GX(18)
+#undef LBM_GX
+    } else {
+#define LBM_GX(S)                                                                     \
+    {                                                                                 \
+        R a = ((R)lbm_ex(S) - vx) * fx;                                               \
+        a = a + ((R)lbm_ey(S) - vy) * fy;                                             \
+        a = a + ((R)lbm_ez(S) - vz) * fz;                                             \
+        G[S] = (R)lbm_w(S) * conv(a, lbm_edot<S, R>(vx, vy, vz) * lbm_edot<S, R>(fx, fy, fz)); \
+    }
+        LBM_GX(0) LBM_GX(1) LBM_GX(2) LBM_GX(3) LBM_GX(4) LBM_GX(5) LBM_GX(6) LBM_GX(7) LBM_GX(8) LBM_GX(9)
+        LBM_GX(10) LBM_GX(11) LBM_GX(12) LBM_GX(13) LBM_GX(14) LBM_GX(15) LBM_GX(16) LBM_GX(17) LBM_GX(18)
+#undef LBM_GX
     }
 }
 
@@ -294,7 +355,7 @@ __device__ __forceinline__ void velocity(R& vx, R& vy, R& vz, R rho, const SpCon
 // F holds f - w and r is rho - 1 (moment 0 of M (f - w)).
 // FAST (deviation-form kernels): pair-form transforms and FMA relaxation; the
 // reference-arithmetic kernels keep the term-by-term order (FAST = false).
-template <typename R, bool FORCE, bool FAST = false>
+template <typename R, int FORCE, bool FAST = false>
 __device__ __forceinline__ void collide_sp(R* F, R r, R vx, R vy, R vz, const SpConsts<R>& C) {
     R m[19];
     if constexpr (FAST) mrt_moments_fast<R>(F, m);
@@ -341,26 +402,8 @@ __device__ __forceinline__ void collide_sp(R* F, R r, R vx, R vy, R vz, const Sp
         m[14] = lbm_fma<R>(kd9, lbm_fma<R>(vy, fz, vz * fy), m[14]);
         m[15] = lbm_fma<R>(kd9, lbm_fma<R>(vx, fz, vz * fx), m[15]);
     } else if constexpr (FORCE) {
-        const R fx = C.fext[0], fy = C.fext[1], fz = C.fext[2];
         R G[19];
-#pragma unroll
-        for (int l = 0; l < 19; ++l) {
-            R a = ((R)lbm_ex(l) - vx) * fx;
-            a = a + ((R)lbm_ey(l) - vy) * fy;
-            a = a + ((R)lbm_ez(l) - vz) * fz;
-            R eu, ef;
-            switch (l) {
-#define LBM_EU(S) case S: eu = lbm_edot<S, R>(vx, vy, vz); ef = lbm_edot<S, R>(fx, fy, fz); break;
-                LBM_EU(0) LBM_EU(1) LBM_EU(2) LBM_EU(3) LBM_EU(4) LBM_EU(5) LBM_EU(6) LBM_EU(7) LBM_EU(8) LBM_EU(9)
-                LBM_EU(10) LBM_EU(11) LBM_EU(12) LBM_EU(13) LBM_EU(14) LBM_EU(15) LBM_EU(16) LBM_EU(17) LBM_EU(18)
-#undef LBM_EU
-            }
-            R g;
-            if (C.guo == 0) g = a / (R)3.0 + (eu * ef) / (R)9.0;   // class (SP:236)
-            else if (C.guo == 1) g = a + eu * ef;                  // scripts (TP:246)
-            else g = (R)3.0 * a + (R)9.0 * (eu * ef);              // standard Guo, c_s^2 = 1/3
-            G[l] = (R)lbm_w(l) * g;
-        }
+        guo_dense<R, FORCE>(G, vx, vy, vz, C.fext, C.guo);
         R fg[19];
         mrt_moments<R>(G, fg);
 #pragma unroll

@@ -67,7 +67,7 @@ namespace {
 using namespace lbmk;
 
 // Macros, collision and store of node n (faces done); ref: its reference density.
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 __device__ __forceinline__ void sp_collide_node(typename Codec<STORE>::R* F, int n, bool pressure_face,
                                                 typename Codec<STORE>::R ref,
                                                 const SpConsts<typename Codec<STORE>::R>& C,
@@ -85,14 +85,7 @@ __device__ __forceinline__ void sp_collide_node(typename Codec<STORE>::R* F, int
     for (int s = 1; s < 19; ++s) r = r + F[s];
     const R rho = Cd::DEV ? (R)1 + r : r;
     R vx = vsum<0>(F), vy = vsum<1>(F), vz = vsum<2>(F);
-    vx = vx / rho;
-    vy = vy / rho;
-    vz = vz / rho;
-    if constexpr (FORCE) {
-        vx = vx + C.fhalf[0] / rho;
-        vy = vy + C.fhalf[1] / rho;
-        vz = vz + C.fhalf[2] / rho;
-    }
+    velocity<R, FORCE>(vx, vy, vz, rho, C.fhalf);
     if (pressure_face) {
         vprev[n] = vx;
         vprev[np + n] = vy;
@@ -110,7 +103,7 @@ __device__ __forceinline__ void sp_collide_node(typename Codec<STORE>::R* F, int
 }
 
 // Everything after the gather: faces, macros, collision and store of node n.
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 __device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int n, int i, int j, int k,
                                                const SpConsts<typename Codec<STORE>::R>& C,
                                                typename Codec<STORE>::T* __restrict__ fout,
@@ -129,7 +122,7 @@ __device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int 
                                           lbm_ref_at(sp_ref(C), i), C, fout, vprev, rho_out, v_out);
 }
 
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1
                                            : Codec<STORE>::RHOREF ? (FORCE ? LBM_SP_MINBLOCKS_16F : LBM_SP_MINBLOCKS_16)
                                        : Codec<STORE>::DEV    ? LBM_SP_MINBLOCKS_DEV
@@ -175,18 +168,20 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1
 // links (lbm_links.cuh, 9 bytes a node read in order) instead of coordinates and
 // 18 map lookups.  What that buys is instructions (877 against 1052 per warp of
 // 32 nodes, FP32; 717 against 890, FP32 deviation form) and one dependent load
-// less before the populations.  On the 256^3 pack, MLUPS, map kernel / link kernel:
-// FP32 33.6k / 35.5k, FP32 deviation form 35.1k / 36.1k, FP16 32.2k / 39.9k;
-// 64^3 cavity FP32 30.1k / 34.3k; forced FP32 channel 101 x 67 x 53 19.3k / 21.3k.
-// FP32 then moves 166 B a node at 0.91 of the copy bandwidth (DRAM-bound); the
-// 16-bit storages and the forced FP32 kernel are bound by issue slots.  Two
-// nodes per thread in packed FP32 halve the instructions and were slower (28.0k
-// FP32, 96 registers: half the warps, each living longer), pushing instead of
-// pulling too (19.5k: unaligned stores leave partly written sectors).
+// less before the populations.  256^3 pack, MLUPS, map kernel / links / links with one
+// reciprocal per density instead of three to six IEEE divisions: FP32 33.6k /
+// 35.5k / 36.9k, FP32 deviation form 35.1k / 36.1k / 38.7k, FP16 32.2k / 39.9k /
+// 40.1k; 64^3 cavity FP32 30.1k / 34.3k / 33.7k (launch-bound); channel 101 x 67 x 53,
+// FP32 forced along x 19.3k / 21.3k / 28.7k (with the x-only Guo term).
+// FP32 then moves 166 B a node at 0.93 of the copy bandwidth (DRAM-bound); the
+// 16-bit storages are bound by issue slots (87% of them used).  Two nodes per
+// thread in packed FP32 halve the instructions and were slower (28.0k FP32, 96
+// registers: half the warps, each living longer), pushing instead of pulling
+// too (19.5k: unaligned stores leave partly written sectors).
 //
 // Resident 128-thread CTAs per SM, measured on the same lattices: 10 (48
-// registers, no spill; FP32 35.5k against 34.4k at 9 and 34.9k at 12, FP16 39.9k
-// against 38.8k at 9 and 39.7k at 11), forced FP32 9 (21.3k against 20.7k at 8).
+// registers, no spill; FP32 36.9k against 36.0k at 9 and 36.2k at 11, FP16 40.6k
+// against 40.3k and 37.4k), forced FP32 reference arithmetic 9 (28.7k; 28.2k at 10).
 #ifndef LBM_LINK_MINBLOCKS
 #define LBM_LINK_MINBLOCKS 10
 #endif
@@ -196,7 +191,7 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1
 constexpr int LINK_THREADS = 128;
 
 // REF: 16-bit storage against a reference density that is not 0 everywhere.
-template <int STORE, bool FORCE, bool MACROS, bool REF>
+template <int STORE, int FORCE, bool MACROS, bool REF>
 __global__ void __launch_bounds__(LINK_THREADS, FORCE && !Codec<STORE>::DEV ? LBM_LINK_MINBLOCKS_F : LBM_LINK_MINBLOCKS)
     sp_link_kernel(const __grid_constant__ SpConsts<float> C, const typename Codec<STORE>::T* f_prev,
                    typename Codec<STORE>::T* __restrict__ fout, const __grid_constant__ LbmLinks L,
@@ -354,7 +349,7 @@ __device__ __forceinline__ void spt_next(const SptArgs& A, int nx, int ny, int n
         for (int pz = 0; pz < 3; ++pz) spt_bulk(s_map + pz * A.plane, map + first[pz], pbytes[pz], bar);
 }
 
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 __global__ void __launch_bounds__(SPT, STORE == LBM_STORE_F64 ? 1
                                        : Codec<STORE>::RHOREF ? (FORCE ? LBM_SP_MINBLOCKS_16F : LBM_SP_MINBLOCKS_16)
                                        : Codec<STORE>::DEV    ? LBM_SP_MINBLOCKS_DEV
@@ -451,7 +446,7 @@ __global__ void __launch_bounds__(SPT, STORE == LBM_STORE_F64 ? 1
 // memory with the bulk-copy engine; coordinates and map never change, so the
 // copies are made before griddepcontrol.wait and overlap the previous step's
 // drain for the CTAs resident by then.
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 __global__ void __launch_bounds__(SPT, STORE == LBM_STORE_F64 ? 1
                                        : Codec<STORE>::RHOREF ? (FORCE ? LBM_SP_MINBLOCKS_16F : LBM_SP_MINBLOCKS_16)
                                        : Codec<STORE>::DEV    ? LBM_SP_MINBLOCKS_DEV
@@ -550,7 +545,7 @@ size_t spt_smem_bytes(int nx) { return SPT_HDR + SPT_STAGES * (SPT * 4 + 3 * (si
 
 // Initial populations: F = feq(rho, v), then one collision with (rho, v)
 // (init SP:160-170 followed by the first step's colission).
-template <int STORE, bool FORCE>
+template <int STORE, int FORCE>
 __global__ void sp_init_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C,
                                typename Codec<STORE>::T* __restrict__ fout, const float* __restrict__ rho_in,
                                const float* __restrict__ v_in, typename Codec<STORE>::R* __restrict__ vprev,
@@ -592,7 +587,7 @@ __global__ void sp_gather_kernel(const __grid_constant__ SpConsts<float> C, cons
     for (int s = 0; s < 19; ++s) out[32 * s] = F[s];
 }
 
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 int launch_step(LbmHandle* h, const SpConsts<typename Codec<STORE>::R>& C, int grid) {
     using T = typename Codec<STORE>::T;
     using R = typename Codec<STORE>::R;
@@ -615,7 +610,7 @@ int launch_step(LbmHandle* h, const SpConsts<typename Codec<STORE>::R>& C, int g
     return lbm_cuda_check(h, e != cudaSuccess ? e : cudaGetLastError(), "sp_step_kernel launch");
 }
 
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 int launch_tile(LbmHandle* h, const SpConsts<typename Codec<STORE>::R>& C, const SptArgs& A, int grid, size_t smem) {
     using T = typename Codec<STORE>::T;
     using R = typename Codec<STORE>::R;
@@ -655,7 +650,7 @@ int launch_tile(LbmHandle* h, const SpConsts<typename Codec<STORE>::R>& C, const
 }
 
 // Resident CTAs of the staged kernel on the whole device (its persistent grid).
-template <int STORE, bool FORCE>
+template <int STORE, int FORCE>
 int tile_grid(LbmHandle* h, size_t smem) {
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sp_tile_kernel<STORE, FORCE, false>, SPT, smem) !=
@@ -689,7 +684,7 @@ int run_tiles(LbmHandle* h, int32_t n, bool macros_last) {
     return LBM_OK;
 }
 
-template <int STORE, bool FORCE, bool MACROS, bool REF>
+template <int STORE, int FORCE, bool MACROS, bool REF>
 int launch_link(LbmHandle* h, const SpConsts<float>& C) {
     using T = typename Codec<STORE>::T;
     const T* fin = (const T*)h->d_f[h->cur];
@@ -711,7 +706,7 @@ int launch_link(LbmHandle* h, const SpConsts<float>& C) {
     return lbm_cuda_check(h, e != cudaSuccess ? e : cudaGetLastError(), "sp_link_kernel launch");
 }
 
-template <int STORE, bool FORCE, bool REF>
+template <int STORE, int FORCE, bool REF>
 int run_links_t(LbmHandle* h, int32_t n, bool macros_last) {
     SpConsts<float> C = sp_make_consts<float>(h);
     for (int32_t it = 0; it < n; ++it) {
@@ -728,11 +723,14 @@ int run_links(LbmHandle* h, int32_t n, bool macros_last) {
     if constexpr (Codec<STORE>::RHOREF) {
         const SpConsts<float> C = sp_make_consts<float>(h);
         if (C.ref_a != 0.0f || C.ref_b != 0.0f)
-            return h->force ? run_links_t<STORE, true, true>(h, n, macros_last)
-                            : run_links_t<STORE, false, true>(h, n, macros_last);
+            return h->force ? run_links_t<STORE, FORCE_ANY, true>(h, n, macros_last)
+                            : run_links_t<STORE, FORCE_NONE, true>(h, n, macros_last);
     }
-    return h->force ? run_links_t<STORE, true, false>(h, n, macros_last)
-                    : run_links_t<STORE, false, false>(h, n, macros_last);
+    // (the deviation form has the Guo term in closed form: one kernel for every force)
+    if constexpr (!Codec<STORE>::DEV)
+        if (force_kind(h) == FORCE_X) return run_links_t<STORE, FORCE_X, false>(h, n, macros_last);
+    return h->force ? run_links_t<STORE, FORCE_ANY, false>(h, n, macros_last)
+                    : run_links_t<STORE, FORCE_NONE, false>(h, n, macros_last);
 }
 
 template <int STORE>

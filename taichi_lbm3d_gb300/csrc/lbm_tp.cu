@@ -203,7 +203,7 @@ __device__ __forceinline__ void recolour_amounts(R rr, R rb, R vx, R vy, R vz, R
 }
 
 // Two-phase MRT collision (TP:302-344) of F in place.
-template <typename R, bool FORCE, bool FAST>
+template <typename R, int FORCE, bool FAST>
 __device__ __forceinline__ void collide_tp(R* F, R r, R vx, R vy, R vz, R cc, R n0, R n1, R n2, R sv, R so,
                                            const TpConsts<R>& T) {
     R m[19];
@@ -233,22 +233,8 @@ __device__ __forceinline__ void collide_tp(R* F, R r, R vx, R vy, R vz, R cc, R 
         else m[s] = m[s] - S * (m[s] - meq[s]);
     }
     if constexpr (FORCE) {
-        const R fx = T.sp.fext[0], fy = T.sp.fext[1], fz = T.sp.fext[2];
         R G[19];
-#pragma unroll
-        for (int l = 0; l < 19; ++l) {
-            R a = ((R)lbm_ex(l) - vx) * fx;
-            a = a + ((R)lbm_ey(l) - vy) * fy;
-            a = a + ((R)lbm_ez(l) - vz) * fz;
-            R eu, ef;
-            switch (l) {
-#define LBM_EU(S) case S: eu = lbm_edot<S, R>(vx, vy, vz); ef = lbm_edot<S, R>(fx, fy, fz); break;
-                LBM_EU(0) LBM_EU(1) LBM_EU(2) LBM_EU(3) LBM_EU(4) LBM_EU(5) LBM_EU(6) LBM_EU(7) LBM_EU(8) LBM_EU(9)
-                LBM_EU(10) LBM_EU(11) LBM_EU(12) LBM_EU(13) LBM_EU(14) LBM_EU(15) LBM_EU(16) LBM_EU(17) LBM_EU(18)
-#undef LBM_EU
-            }
-            G[l] = (R)lbm_w(l) * (a + eu * ef);  // GuoF, TP:242-248
-        }
+        guo_dense<R, FORCE>(G, vx, vy, vz, T.sp.fext, 1);   // GuoF, TP:242-248
         R fg[19];
         if constexpr (FAST) mrt_moments_fast<R>(G, fg);
         else mrt_moments<R>(G, fg);
@@ -266,7 +252,7 @@ __device__ __forceinline__ void collide_tp(R* F, R r, R vx, R vy, R vz, R cc, R 
 
 // Everything B does after the macros: recolouring amounts, collision, and what
 // the next launch A pulls.
-template <int STORE, bool FORCE>
+template <int STORE, int FORCE>
 __device__ __forceinline__ void tp_collide_and_store(typename Codec<STORE>::R* F, typename Codec<STORE>::R r,
                                                      typename Codec<STORE>::R vx, typename Codec<STORE>::R vy,
                                                      typename Codec<STORE>::R vz, int n,
@@ -407,7 +393,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : LBM_TP_MINBLOCKS_A) 
 }
 
 // ---------------------------------------------------------------- launch B
-template <int STORE, bool FORCE, bool MACROS>
+template <int STORE, int FORCE, bool MACROS>
 __global__ void __launch_bounds__(128, STORE == LBM_STORE_F64 ? 2 : LBM_TP_MINBLOCKS_B) tp_flow_kernel(
     const __grid_constant__ TpConsts<typename Codec<STORE>::R> T, const typename Codec<STORE>::T* f_prev,
     typename Codec<STORE>::T* __restrict__ fout, const int32_t* __restrict__ map, const uint32_t* __restrict__ coord,
@@ -444,7 +430,7 @@ __global__ void __launch_bounds__(128, STORE == LBM_STORE_F64 ? 2 : LBM_TP_MINBL
     for (int s = 1; s < 19; ++s) r = r + F[s];
     const R rho = Cd::DEV ? (R)1 + r : r;
     R vx = vsum<0>(F), vy = vsum<1>(F), vz = vsum<2>(F);
-    velocity<R, FORCE>(vx, vy, vz, rho, C);
+    velocity<R, FORCE>(vx, vy, vz, rho, C.fhalf);
     if (MACROS) rho_out[n] = rho;
     if (MACROS || (K.bits & LBM_LINK_PRESSURE)) {
         v[n] = vx;
@@ -470,7 +456,7 @@ __global__ void tp_psi_kernel(const __grid_constant__ TpConsts<typename Codec<ST
     psi[n] = (typename Codec<STORE>::R)psi0[lbm_pi(pc) + (int64_t)T.sp.nx * (lbm_pj(pc) + (int64_t)T.sp.ny * lbm_pk(pc))];
 }
 
-template <int STORE, bool FORCE>
+template <int STORE, int FORCE>
 __global__ void tp_init_kernel(const __grid_constant__ TpConsts<typename Codec<STORE>::R> T,
                                typename Codec<STORE>::T* __restrict__ fout, const int32_t* __restrict__ map,
                                const uint32_t* __restrict__ coord, typename Codec<STORE>::R* __restrict__ v,
@@ -537,7 +523,7 @@ int tp_init_t(LbmHandle* h) {
     h->cur = 0;
     const int grid = (int)((h->n_fluid + h->block - 1) / h->block);
     tp_psi_kernel<STORE><<<grid, h->block, 0, h->stream>>>(T, h->d_coord, h->d_psi0, (R*)h->d_psi);
-    auto k = h->force ? tp_init_kernel<STORE, true> : tp_init_kernel<STORE, false>;
+    auto k = h->force ? tp_init_kernel<STORE, FORCE_ANY> : tp_init_kernel<STORE, FORCE_NONE>;
     k<<<grid, h->block, 0, h->stream>>>(T, (Tt*)h->d_f[0], h->d_map, h->d_coord, (R*)h->d_v, (R*)h->d_rho,
                                         (R*)h->d_rr, (R*)h->d_rb, (const R*)h->d_psi, (ColourRec<R>*)h->d_crec,
                                         (R*)h->d_pull_vz, (R*)h->d_cs);
@@ -546,7 +532,7 @@ int tp_init_t(LbmHandle* h) {
     return rc;
 }
 
-template <int STORE, bool FORCE>
+template <int STORE, int FORCE>
 int tp_steps_t(LbmHandle* h, int32_t nsteps, bool macros_last) {
     using R = typename Codec<STORE>::R;
     using Tt = typename Codec<STORE>::T;
@@ -574,7 +560,11 @@ int tp_steps_t(LbmHandle* h, int32_t nsteps, bool macros_last) {
 
 template <int STORE>
 int tp_steps(LbmHandle* h, int32_t n, bool macros_last) {
-    return h->force ? tp_steps_t<STORE, true>(h, n, macros_last) : tp_steps_t<STORE, false>(h, n, macros_last);
+    switch (force_kind(h)) {
+    case FORCE_NONE: return tp_steps_t<STORE, FORCE_NONE>(h, n, macros_last);
+    case FORCE_X: return tp_steps_t<STORE, FORCE_X>(h, n, macros_last);
+    }
+    return tp_steps_t<STORE, FORCE_ANY>(h, n, macros_last);
 }
 
 }  // namespace

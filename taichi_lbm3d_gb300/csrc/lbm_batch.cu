@@ -69,9 +69,9 @@ using namespace lbmk;
 // loaded while the step before drains.  Eight subvolumes of edges 48 to 160 (4.07 M
 // fluid nodes, body force), MLUPS, against a persistent grid whose CTAs claimed
 // 1024-node tiles from a counter and looked sources up in the dense maps: FP16
-// 38.0k / 32.0k, FP32 deviation form 36.3k / 30.9k, FP32 23.5k / 20.2k.  Bound by
+// 42.0k / 32.0k, FP32 deviation form 37.9k / 30.9k, FP32 31.0k / 20.2k.  Bound by
 // issue slots as the single-lattice kernel.  Tiles of 64 and 128 threads run
-// alike (38.1k, 38.0k FP16), of 256 36.0k.
+// alike, of 256 5% slower.
 template <int STORE, int FORCE, bool CHECK>
 __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Codec<STORE>::DEV ? 4 : 5)
     batch_step_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C, const BatchTile* __restrict__ tiles,
@@ -80,6 +80,8 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Co
                       double* __restrict__ partial) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
+    constexpr bool RAW = Cd::SCALE != 1;
+    constexpr int SC = RAW ? Cd::SCALE : 1;
     __shared__ double s_red[32];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int4 t4 = __ldg(reinterpret_cast<const int4*>(tiles + blockIdx.x));
@@ -99,16 +101,18 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Co
     double acc = 0.0;
     if (live) {
         R F[19];
-        LinkGather<STORE, false>::all(F, fin, L, K, n, none);
+        LinkGather<STORE, false, RAW>::all(F, fin, L, K, n, none);
         R r = F[0];
 #pragma unroll
         for (int s = 1; s < 19; ++s) r = r + F[s];
-        const R rho = Cd::DEV ? (R)1 + r : r;
+        const R rho = Cd::DEV ? (R)SC + r : r;   // times SC, as the sums over F
         R vx = vsum<0>(F), vy = vsum<1>(F), vz = vsum<2>(F);
-        velocity<R, FORCE>(vx, vy, vz, rho, C.fhalf);
+        const R fhalf[3] = {C.fhalf[0] * (R)SC, C.fhalf[1] * (R)SC, C.fhalf[2] * (R)SC};
+        velocity<R, FORCE>(vx, vy, vz, rho, fhalf);
         if constexpr (CHECK) acc += (double)vx;
-        collide_sp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, C);
-        store_node<STORE>(F, out, n, (R)0, seed);
+        collide_sp<R, FORCE, Cd::DEV, SC>(F, r, vx, vy, vz, C);
+        if constexpr (RAW) store_node_raw<STORE>(F, out, n, (R)0, seed);
+        else store_node<STORE>(F, out, n, (R)0, seed);
     }
     if constexpr (CHECK) {
         for (int off = 16; off > 0; off >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, off);

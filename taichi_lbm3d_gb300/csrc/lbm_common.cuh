@@ -154,28 +154,37 @@ __device__ __forceinline__ uint32_t lbm_sr_bits(uint32_t h) {
     return h * (0x2545F491u + 2u * 0x9E37u * (uint32_t)S);
 }
 
+// SCALE: the link steps of the FP16 codec compute on f' * 2^16, as stored, instead
+// of scaling each of the 19 values back and forth: a power of two commutes with
+// every rounding of the linear and quadratic terms, so the stored bits are the
+// same (raw / enc_sr_raw; everything else uses dec / enc_sr).
 template <int STORE> struct Codec;
 template <> struct Codec<LBM_STORE_F32> {
     using T = float; using R = float;
     static constexpr bool DEV = false, RHOREF = false;
+    static constexpr int SCALE = 1;
     template <int S> static __device__ __forceinline__ R dec(T x) { return x; }
     template <int S> static __device__ __forceinline__ T enc(R f) { return f; }
 };
 template <> struct Codec<LBM_STORE_F64> {
     using T = double; using R = double;
     static constexpr bool DEV = false, RHOREF = false;
+    static constexpr int SCALE = 1;
     template <int S> static __device__ __forceinline__ R dec(T x) { return x; }
     template <int S> static __device__ __forceinline__ T enc(R f) { return f; }
 };
 template <> struct Codec<LBM_STORE_F32_DEV> {
     using T = float; using R = float;
     static constexpr bool DEV = true, RHOREF = false;
+    static constexpr int SCALE = 1;
     template <int S> static __device__ __forceinline__ R dec(T x) { return x; }
     template <int S> static __device__ __forceinline__ T enc(R f) { return f; }
 };
 template <> struct Codec<LBM_STORE_F16_DEV> {
     using T = __half; using R = float;
     static constexpr bool DEV = true, RHOREF = true;
+    static constexpr int SCALE = 65536;
+    template <int S> static __device__ __forceinline__ R raw(T x) { return __half2float(x); }
     template <int S> static __device__ __forceinline__ R dec(T x) { return __half2float(x) * (1.0f / 65536.0f); }
     template <int S> static __device__ __forceinline__ T enc(R g) { return __float2half_rn(g * 65536.0f); }
     // 13 bits below the FP16 mantissa (exact for FP16 normals; FP16
@@ -184,10 +193,19 @@ template <> struct Codec<LBM_STORE_F16_DEV> {
         const uint32_t u = __float_as_uint(g * 65536.0f) + (lbm_sr_bits<S>(h) >> 19);
         return __float2half_rz(__uint_as_float(u));
     }
+    // two directions of a value already scaled, converted together (low half: S)
+    template <int S> static __device__ __forceinline__ uint32_t enc_sr_raw2(R g0, R g1, uint32_t h) {
+        const float a = __uint_as_float(__float_as_uint(g0) + (lbm_sr_bits<S>(h) >> 19));
+        const float b = __uint_as_float(__float_as_uint(g1) + (lbm_sr_bits<S + 1>(h) >> 19));
+        uint32_t w;
+        asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(b), "f"(a));
+        return w;
+    }
 };
 template <> struct Codec<LBM_STORE_BF16_DEV> {
     using T = __nv_bfloat16; using R = float;
     static constexpr bool DEV = true, RHOREF = true;
+    static constexpr int SCALE = 1;
     template <int S> static __device__ __forceinline__ R dec(T x) { return __bfloat162float(x); }
     template <int S> static __device__ __forceinline__ T enc(R g) { return __float2bfloat16_rn(g); }
     template <int S> static __device__ __forceinline__ T enc_sr(R g, uint32_t h) {

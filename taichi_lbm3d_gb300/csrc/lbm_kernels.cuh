@@ -231,6 +231,33 @@ __device__ __forceinline__ void store_node(const typename Codec<STORE>::R* F, ty
     }
 }
 
+// The same for values in the codec's own scale (Codec::SCALE); ref_own scaled.
+template <int STORE>
+__device__ __forceinline__ void store_node_raw(const typename Codec<STORE>::R* F, typename Codec<STORE>::T* __restrict__ fout,
+                                               int n, typename Codec<STORE>::R ref_own, uint32_t seed) {
+    using Cd = Codec<STORE>;
+    using R = typename Cd::R;
+    if constexpr (LBM_SR != 0) {
+        uint16_t* out = reinterpret_cast<uint16_t*>(fout + lbm_eoff32(n));
+        const uint32_t h = lbm_sr_hash((uint32_t)n, seed);
+        auto g = [&](int s) { return lbm_fma<R>(-(R)lbm_w(s), ref_own, F[s]); };
+        out[0] = (uint16_t)Cd::template enc_sr_raw2<0>(g(0), (R)0, h);
+#define LBM_S(S)                                                               \
+    {                                                                          \
+        const uint32_t w = Cd::template enc_sr_raw2<S>(g(S), g(S + 1), h);     \
+        out[32 * S] = (uint16_t)w;                                             \
+        out[32 * S + 32] = (uint16_t)(w >> 16);                                \
+    }
+        LBM_S(1) LBM_S(3) LBM_S(5) LBM_S(7) LBM_S(9) LBM_S(11) LBM_S(13) LBM_S(15) LBM_S(17)
+#undef LBM_S
+    } else {
+        R f[19];
+#pragma unroll
+        for (int s = 0; s < 19; ++s) f[s] = F[s] * (R)(1.0 / Cd::SCALE);
+        store_node<STORE>(f, fout, n, ref_own * (R)(1.0 / Cd::SCALE), seed);
+    }
+}
+
 // v component sums: sum_s e_s[c] F[s] with zero terms dropped (SP:382-383).
 template <int C, typename R>
 __device__ __forceinline__ R vsum(const R* F) {
@@ -355,19 +382,21 @@ __device__ __forceinline__ void guo_dense(R* G, R vx, R vy, R vz, const R (&fext
 // F holds f - w and r is rho - 1 (moment 0 of M (f - w)).
 // FAST (deviation-form kernels): pair-form transforms and FMA relaxation; the
 // reference-arithmetic kernels keep the term-by-term order (FAST = false).
-template <typename R, int FORCE, bool FAST = false>
+// SC: F and r hold SC (a power of two) times their values (FAST only).
+template <typename R, int FORCE, bool FAST = false, int SC = 1>
 __device__ __forceinline__ void collide_sp(R* F, R r, R vx, R vy, R vz, const SpConsts<R>& C) {
     R m[19];
     if constexpr (FAST) mrt_moments_fast<R>(F, m);
     else mrt_moments<R>(F, m);
-    const R uu = lbm_usq(vx, vy, vz);
+    const R ux = SC == 1 ? vx : vx * (R)SC, uy = SC == 1 ? vy : vy * (R)SC, uz = SC == 1 ? vz : vz * (R)SC;
     R meq[19];
 #pragma unroll
     for (int s = 0; s < 19; ++s) meq[s] = (R)0;
-    meq[0] = r; meq[3] = vx; meq[5] = vy; meq[7] = vz; meq[1] = uu;
-    meq[9] = (((R)2 * vx) * vx - vy * vy) - vz * vz;
-    meq[11] = vy * vy - vz * vz;
-    meq[13] = vx * vy; meq[14] = vy * vz; meq[15] = vx * vz;
+    (void)r;   // moments 0, 3, 5, 7 are conserved
+    meq[1] = (ux * vx + uy * vy) + uz * vz;
+    meq[9] = (((R)2 * ux) * vx - uy * vy) - uz * vz;
+    meq[11] = uy * vy - uz * vz;
+    meq[13] = ux * vy; meq[14] = uy * vz; meq[15] = ux * vz;
 #pragma unroll
     for (int s = 0; s < 19; ++s) {
         const int kd = lbm_skind(s);
@@ -384,7 +413,7 @@ __device__ __forceinline__ void collide_sp(R* F, R r, R vx, R vy, R vz, const Sp
         // gd (4 ux Fx - 2 uy Fy - 2 uz Fz) / 9, moment 11: 2/9 gd (uy Fy - uz Fz),
         // moments 13, 14, 15: gd (ua Fb + ub Fa) / 9; the others vanish.  Moments
         // 0, 3, 5, 7 are conserved (S = 0); 1, 9, 11, 13-15 relax with s_v.
-        const R fx = C.fext[0], fy = C.fext[1], fz = C.fext[2];
+        const R fx = C.fext[0] * (R)SC, fy = C.fext[1] * (R)SC, fz = C.fext[2] * (R)SC;
         const R gc = C.gc, gd = C.gd;
         const R ksv = (R)1 - (R)0.5 * C.sv;
         const R uf = lbm_fma<R>(vz, fz, lbm_fma<R>(vy, fy, vx * fx));

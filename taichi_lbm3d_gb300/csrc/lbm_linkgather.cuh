@@ -84,6 +84,11 @@ struct LinkRef {
         xm = inside ? at - ref.b : lbm_fma<R>(ref.b, (R)(i == 0 ? nx - 1 : i - 1), ref.a);
         xp = inside ? at + ref.b : lbm_fma<R>(ref.b, (R)(i == nx - 1 ? 0 : i + 1), ref.a);
     }
+    __device__ __forceinline__ void scale(R k) {
+        at = at * k;
+        xm = xm * k;
+        xp = xp * k;
+    }
     template <int S>
     __device__ __forceinline__ R of() const {
         return lbm_ex(S) > 0 ? xm : (lbm_ex(S) < 0 ? xp : at);
@@ -93,16 +98,22 @@ struct LinkRef {
 // All of a node's pulled populations.  Direction s and its opposite are
 // neighbours in the slot order, so the own opposite slot is the own slot s moved
 // by one: both candidates of the load share the immediate offset of slot s.
-template <int STORE, bool REF>
+// RAW: in the codec's own scale (Codec::SCALE), rx scaled alike.
+template <int STORE, bool REF, bool RAW = false>
 struct LinkGather {
     using Cd = Codec<STORE>;
     using T = typename Cd::T;
     using R = typename Cd::R;
     template <int S>
+    static __device__ __forceinline__ R get(T x) {
+        if constexpr (RAW) return Cd::template raw<S>(x);
+        else return Cd::template dec<S>(x);
+    }
+    template <int S>
     static __device__ __forceinline__ void one(R* F, const T* fin, int own, const NodeLinks& K, int n, const LinkRef<R>& rx) {
         const bool bounce = K.bits >> S & 1u;
         const int a = bounce ? own + 32 * (lbm_lr(S) - S) : lbm_eoff32(K.template source<S>(n));
-        F[S] = Cd::template dec<S>(fin[a + 32 * S]);
+        F[S] = get<S>(fin[a + 32 * S]);
         if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), bounce ? rx.at : rx.template of<S>(), F[S]);
     }
     // Explicit sources of the links that the node word cannot express; a warp
@@ -115,7 +126,7 @@ struct LinkGather {
     {                                                                                         \
         const int src = __ldg(rec + S);                                                       \
         if (src >= 0) {                                                                       \
-            F[S] = Cd::template dec<S>(fin[lbm_eoff32(src) + 32 * S]);                        \
+            F[S] = get<S>(fin[lbm_eoff32(src) + 32 * S]);                        \
             if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), rx.template of<S>(), F[S]);     \
         }                                                                                     \
     }
@@ -125,7 +136,7 @@ struct LinkGather {
     static __device__ __forceinline__ void all(R* F, const T* fin, const LbmLinks& L, const NodeLinks& K, int n,
                                                const LinkRef<R>& rx) {
         const int own = lbm_eoff32(n);
-        F[0] = Cd::template dec<0>(fin[own]);
+        F[0] = get<0>(fin[own]);
         if constexpr (REF) F[0] = lbm_fma<R>((R)lbm_w(0), rx.at, F[0]);
 #define LBM_G(S) one<S>(F, fin, own, K, n, rx);
         LBM_ALL_DIRS(LBM_G)

@@ -67,7 +67,8 @@ namespace {
 using namespace lbmk;
 
 // Macros, collision and store of node n (faces done); ref: its reference density.
-template <int STORE, int FORCE, bool MACROS>
+// RAW: F and ref in the codec's own scale.
+template <int STORE, int FORCE, bool MACROS, bool RAW = false>
 __device__ __forceinline__ void sp_collide_node(typename Codec<STORE>::R* F, int n, bool pressure_face,
                                                 typename Codec<STORE>::R ref,
                                                 const SpConsts<typename Codec<STORE>::R>& C,
@@ -83,23 +84,26 @@ __device__ __forceinline__ void sp_collide_node(typename Codec<STORE>::R* F, int
     R r = F[0];
 #pragma unroll
     for (int s = 1; s < 19; ++s) r = r + F[s];
-    const R rho = Cd::DEV ? (R)1 + r : r;
+    constexpr int SC = RAW ? Cd::SCALE : 1;
+    const R rho = Cd::DEV ? (R)SC + r : r;   // times SC, as the sums over F
     R vx = vsum<0>(F), vy = vsum<1>(F), vz = vsum<2>(F);
-    velocity<R, FORCE>(vx, vy, vz, rho, C.fhalf);
+    const R fhalf[3] = {C.fhalf[0] * (R)SC, C.fhalf[1] * (R)SC, C.fhalf[2] * (R)SC};
+    velocity<R, FORCE>(vx, vy, vz, rho, fhalf);
     if (pressure_face) {
         vprev[n] = vx;
         vprev[np + n] = vy;
         vprev[2 * np + n] = vz;
     }
     if constexpr (MACROS) {
-        rho_out[n] = rho;
+        rho_out[n] = rho * (R)(1.0 / SC);
         v_out[n] = vx;
         v_out[np + n] = vy;
         v_out[2 * np + n] = vz;
     }
 
-    collide_sp<R, FORCE, Cd::DEV>(F, r, vx, vy, vz, C);
-    store_node<STORE>(F, fout, n, ref, C.seed);
+    collide_sp<R, FORCE, Cd::DEV, SC>(F, r, vx, vy, vz, C);
+    if constexpr (RAW) store_node_raw<STORE>(F, fout, n, ref, C.seed);
+    else store_node<STORE>(F, fout, n, ref, C.seed);
 }
 
 // Everything after the gather: faces, macros, collision and store of node n.
@@ -171,7 +175,7 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1
 // less before the populations.  256^3 pack, MLUPS, map kernel / links / links with one
 // reciprocal per density instead of three to six IEEE divisions: FP32 33.6k /
 // 35.5k / 36.9k, FP32 deviation form 35.1k / 36.1k / 38.7k, FP16 32.2k / 39.9k /
-// 40.1k; 64^3 cavity FP32 30.1k / 34.3k / 33.7k (launch-bound); channel 101 x 67 x 53,
+// 40.6k; 64^3 cavity FP32 30.1k / 34.3k / 33.7k (launch-bound); channel 101 x 67 x 53,
 // FP32 forced along x 19.3k / 21.3k / 28.7k (with the x-only Guo term).
 // FP32 then moves 166 B a node at 0.93 of the copy bandwidth (DRAM-bound); the
 // 16-bit storages are bound by issue slots (87% of them used).  Two nodes per
@@ -207,15 +211,21 @@ __global__ void __launch_bounds__(LINK_THREADS, FORCE && !Codec<STORE>::DEV ? LB
     K.load(L, n);
     int i = 0;
     if constexpr (REF) i = lbm_pi(__ldg(coord + n));
-    const LinkRef<float> rx(sp_ref(C), i, C.nx);
+    constexpr bool RAW = Cd::SCALE != 1;
+    LinkRef<float> rx(sp_ref(C), i, C.nx);
+    if constexpr (RAW) rx.scale((float)Cd::SCALE);
     const auto* fin = wait_previous(f_prev);
     float F[19];
-    LinkGather<STORE, REF>::all(F, fin, L, K, n, rx);
+    LinkGather<STORE, REF, RAW>::all(F, fin, L, K, n, rx);
     if (K.bits & LBM_LINK_FACE) {
         const uint32_t pc = __ldg(coord + n);
+        if constexpr (Cd::SCALE != 1)
+            for (int s = 0; s < 19; ++s) F[s] = F[s] * (float)(1.0 / Cd::SCALE);
         apply_faces<float, Cd::DEV>(F, lbm_pi(pc), lbm_pj(pc), lbm_pk(pc), n, C, map, vprev);
+        if constexpr (Cd::SCALE != 1)
+            for (int s = 0; s < 19; ++s) F[s] = F[s] * (float)Cd::SCALE;
     }
-    sp_collide_node<STORE, FORCE, MACROS>(F, n, K.bits & LBM_LINK_PRESSURE, rx.at, C, fout, vprev, rho_out, v_out);
+    sp_collide_node<STORE, FORCE, MACROS, RAW>(F, n, K.bits & LBM_LINK_PRESSURE, rx.at, C, fout, vprev, rho_out, v_out);
 }
 
 // ------------------------------------------------------------ staged step

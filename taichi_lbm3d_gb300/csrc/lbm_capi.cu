@@ -338,8 +338,12 @@ int lbm_set_grey(LbmHandle* h, const double* ns) {
         dev_free(h->d_gstale);
         return rc;
     }
+    if (!h->d_links) {   // FP64
+        const LbmLinkLattice lat{h->p.nx, h->p.ny, h->p.nz, h->n_fluid, 0, 0};
+        rc = links_build(h, &lat, 1);
+        if (rc) return rc;
+    }
     h->grey = true;
-    if (!h->l2_persist) l2_persist_map(h);   // the grey step reads the map
     return LBM_OK;
 }
 

@@ -126,34 +126,41 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Co
     }
 }
 
-// rho and v of one subvolume's nodes from its current populations (the
-// macroscopic step of the next update, without collision or store).
+// rho [cell] and v [cell][3] of one subvolume from its current populations (the
+// macroscopic step of the next update, without collision or store); solid 1 and 0.
 template <int STORE, bool FORCE>
 __global__ void batch_macros_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C, BatchSub sd,
                                     const typename Codec<STORE>::T* __restrict__ fin, const int32_t* __restrict__ map,
-                                    const uint32_t* __restrict__ coord, float* __restrict__ out) {
+                                    float* __restrict__ rho_out, float* __restrict__ v_out) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
-    const int a = blockIdx.x * blockDim.x + threadIdx.x;
-    if (a >= sd.n_fluid) return;
-    const uint32_t pc = __ldg(coord + sd.node_begin + a);
-    R F[19];
-    gather_node<STORE>(F, sub_pop(fin, sd.node_begin), map + sd.map_off, a, sd.nx, sd.ny, sd.nz, lbm_pi(pc), lbm_pj(pc),
-                       lbm_pk(pc));
-    R r = F[0];
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= (int64_t)sd.nx * sd.ny * sd.nz) return;
+    const int32_t* smap = map + sd.map_off;
+    const int n = smap[c];
+    float o[4] = {1.0f, 0.0f, 0.0f, 0.0f};
+    if (n >= 0) {
+        const int i = (int)(c % sd.nx), j = (int)(c / sd.nx % sd.ny), k = (int)(c / ((int64_t)sd.nx * sd.ny));
+        R F[19];
+        gather_node<STORE>(F, sub_pop(fin, sd.node_begin), smap, n, sd.nx, sd.ny, sd.nz, i, j, k);
+        R r = F[0];
 #pragma unroll
-    for (int s = 1; s < 19; ++s) r = r + F[s];
-    const R rho = Cd::DEV ? (R)1 + r : r;
-    R vx = vsum<0>(F) / rho, vy = vsum<1>(F) / rho, vz = vsum<2>(F) / rho;
-    if constexpr (FORCE) {
-        vx = vx + C.fhalf[0] / rho;
-        vy = vy + C.fhalf[1] / rho;
-        vz = vz + C.fhalf[2] / rho;
+        for (int s = 1; s < 19; ++s) r = r + F[s];
+        const R rho = Cd::DEV ? (R)1 + r : r;
+        R vx = vsum<0>(F) / rho, vy = vsum<1>(F) / rho, vz = vsum<2>(F) / rho;
+        if constexpr (FORCE) {
+            vx = vx + C.fhalf[0] / rho;
+            vy = vy + C.fhalf[1] / rho;
+            vz = vz + C.fhalf[2] / rho;
+        }
+        o[0] = (float)rho;
+        o[1] = (float)vx;
+        o[2] = (float)vy;
+        o[3] = (float)vz;
     }
-    out[4 * a] = (float)rho;
-    out[4 * a + 1] = (float)vx;
-    out[4 * a + 2] = (float)vy;
-    out[4 * a + 3] = (float)vz;
+    rho_out[c] = o[0];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) v_out[3 * c + d] = o[1 + d];
 }
 
 template <int STORE, bool FORCE>
@@ -245,16 +252,15 @@ int init_t(LbmBatch* b) {
 }
 
 template <int STORE>
-int macros_t(LbmBatch* b, int q, float* d_out) {
+int macros_t(LbmBatch* b, int q, float* rho, float* v) {
     using Cd = Codec<STORE>;
     using R = typename Cd::R;
     LbmHandle* h = &b->h;
     const SpConsts<R> C = sp_make_consts<R>(h);
     const BatchSub sd = b->subs[q];
-    const int grid = (sd.n_fluid + 255) / 256;
+    const int grid = (int)(((int64_t)sd.nx * sd.ny * sd.nz + 127) / 128);
     auto k = h->force ? batch_macros_kernel<STORE, true> : batch_macros_kernel<STORE, false>;
-    if (grid > 0)
-        k<<<grid, 256, 0, h->stream>>>(C, sd, (const typename Cd::T*)h->d_f[0], h->d_map, h->d_coord, d_out);
+    k<<<grid, 128, 0, h->stream>>>(C, sd, (const typename Cd::T*)h->d_f[0], h->d_map, rho, v);
     return lbm_cuda_check(h, cudaGetLastError(), "batch_macros_kernel launch");
 }
 
@@ -564,40 +570,31 @@ int lbm_batch_get_macros(LbmBatch* b, int32_t sub, float* rho, float* v) {
     LbmHandle* h = &b->h;
     cudaSetDevice(h->device);
     const BatchSub sd = b->subs[sub];
-    float* d_out = nullptr;
-    if (cudaMalloc((void**)&d_out, sizeof(float) * 4 * std::max(1, sd.n_fluid)) != cudaSuccess)
-        return batch_err(b, LBM_ENOMEM, "lbm_batch_get_macros: out of device memory");
+    const int64_t nc = (int64_t)sd.nx * sd.ny * sd.nz;
+    // the second population buffer holds nothing between runs of an even number of steps
+    const size_t bytes[2] = {sizeof(float) * (size_t)nc, sizeof(float) * 3 * (size_t)nc};
+    float* own = nullptr;
+    float* d_out = (float*)h->d_f[1];
+    if (bytes[0] + bytes[1] > h->elem * 19 * (size_t)h->np) {
+        if (cudaMalloc((void**)&own, bytes[0] + bytes[1]) != cudaSuccess)
+            return batch_err(b, LBM_ENOMEM, "lbm_batch_get_macros: out of device memory");
+        d_out = own;
+    }
     int rc = 0;
     switch (h->p.storage) {
-    case LBM_STORE_F32: rc = macros_t<LBM_STORE_F32>(b, sub, d_out); break;
-    case LBM_STORE_F16_DEV: rc = macros_t<LBM_STORE_F16_DEV>(b, sub, d_out); break;
-    case LBM_STORE_BF16_DEV: rc = macros_t<LBM_STORE_BF16_DEV>(b, sub, d_out); break;
-    case LBM_STORE_F32_DEV: rc = macros_t<LBM_STORE_F32_DEV>(b, sub, d_out); break;
-    case LBM_STORE_F64: rc = macros_t<LBM_STORE_F64>(b, sub, d_out); break;
+    case LBM_STORE_F32: rc = macros_t<LBM_STORE_F32>(b, sub, d_out, d_out + nc); break;
+    case LBM_STORE_F16_DEV: rc = macros_t<LBM_STORE_F16_DEV>(b, sub, d_out, d_out + nc); break;
+    case LBM_STORE_BF16_DEV: rc = macros_t<LBM_STORE_BF16_DEV>(b, sub, d_out, d_out + nc); break;
+    case LBM_STORE_F32_DEV: rc = macros_t<LBM_STORE_F32_DEV>(b, sub, d_out, d_out + nc); break;
+    case LBM_STORE_F64: rc = macros_t<LBM_STORE_F64>(b, sub, d_out, d_out + nc); break;
     }
-    std::vector<float> tmp(4 * (size_t)sd.n_fluid);
-    if (!rc && sd.n_fluid)
-        rc = lbm_cuda_check(h, cudaMemcpyAsync(tmp.data(), d_out, sizeof(float) * tmp.size(), cudaMemcpyDeviceToHost, h->stream), "copy macros");
-    if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "batch macros");
-    cudaFree(d_out);
-    if (rc) return rc;
-    // scatter to the dense lattice (solid: rho = 1, v = 0) through the host copy of the map
-    const int64_t nc = (int64_t)sd.nx * sd.ny * sd.nz;
-    std::vector<int32_t> map(nc);
-    rc = lbm_cuda_check(h, cudaMemcpy(map.data(), h->d_map + sd.map_off, sizeof(int32_t) * nc, cudaMemcpyDeviceToHost), "copy map");
-    if (rc) return rc;
-    for (int64_t c = 0; c < nc; ++c) {
-        const int32_t nd = map[c];
-        if (nd < 0) {
-            rho[c] = 1.0f;
-            v[3 * c] = v[3 * c + 1] = v[3 * c + 2] = 0.0f;
-        } else {
-            const int64_t a = nd;
-            rho[c] = tmp[4 * a];
-            for (int d = 0; d < 3; ++d) v[3 * c + d] = tmp[4 * a + 1 + d];
-        }
-    }
-    return LBM_OK;
+    void* const host[2] = {rho, v};
+    if (!rc) host_touch(host, bytes, 2);
+    for (int q = 0; q < 2 && !rc; ++q)
+        rc = lbm_cuda_check(h, cudaMemcpyAsync(host[q], d_out + (q ? nc : 0), bytes[q], cudaMemcpyDeviceToHost, h->stream), "copy macros");
+    const int rs = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "batch macros");
+    cudaFree(own);
+    return rc ? rc : rs;
 }
 
 int lbm_batch_get_stream(LbmBatch* b, void** stream) {

@@ -115,23 +115,14 @@ void free_lattice(LbmHandle* h) {
     h->spt_base = 0;
     h->ntile = 0;
     h->tiled = false;
-    dev_free(h->d_f[0]);
-    dev_free(h->d_f[1]);
-    dev_free(h->d_vprev);
-    dev_free(h->d_rho);
-    dev_free(h->d_v);
-    dev_free(h->d_psi);
-    dev_free(h->d_psi0);
-    dev_free(h->d_rr);
-    dev_free(h->d_rb);
-    dev_free(h->d_crec);
-    dev_free(h->d_pull_vz);
-    dev_free(h->d_cs);
+    dev_free(h->d_arena);
+    h->d_f[0] = h->d_f[1] = h->d_vprev = h->d_rho = h->d_v = nullptr;
+    h->d_psi = h->d_rr = h->d_rb = h->d_crec = h->d_pull_vz = h->d_cs = nullptr;
+    h->d_psi0 = nullptr;
+    h->d_red = h->d_red_out = nullptr;
     dev_free(h->d_ns);
     dev_free(h->d_gstale);
     h->grey = false;
-    dev_free(h->d_red);
-    dev_free(h->d_red_out);
     h->device_bytes = 0;
 }
 
@@ -333,27 +324,42 @@ int lbm_set_geometry_strided(LbmHandle* h, const int8_t* solid, int64_t si, int6
     }
     if (rc) { free_lattice(h); return rc; }
     const size_t rbytes = h->f64 ? 8 : 4;
-    rc = rc ? rc : dev_alloc(h, &h->d_f[0], h->elem * 19 * h->np, "f_A");
-    rc = rc ? rc : dev_alloc(h, &h->d_f[1], h->elem * 19 * h->np, "f_B");
-    rc = rc ? rc : dev_alloc(h, &h->d_vprev, rbytes * 3 * h->np, "vprev");
-    rc = rc ? rc : dev_alloc(h, &h->d_rho, rbytes * h->np, "rho");
-    rc = rc ? rc : dev_alloc(h, &h->d_v, rbytes * 3 * h->np, "v");
-    if (!rc && h->p.two_phase) {
-        rc = rc ? rc : dev_alloc(h, &h->d_psi, rbytes * h->np, "psi");
-        rc = rc ? rc : dev_alloc(h, &h->d_psi0, sizeof(float) * h->ncell, "initial psi");
-        rc = rc ? rc : dev_alloc(h, &h->d_rr, rbytes * h->np, "rho_r");
-        rc = rc ? rc : dev_alloc(h, &h->d_rb, rbytes * h->np, "rho_b");
-        rc = rc ? rc : dev_alloc(h, &h->d_crec, rbytes * 4 * h->np, "colour records");
-        rc = rc ? rc : dev_alloc(h, &h->d_pull_vz, rbytes * h->np, "pulled v_z");
-        rc = rc ? rc : dev_alloc(h, &h->d_cs, rbytes * 9 * h->np, "recolouring amounts");
-    }
     h->red_blocks = (int)std::min<int64_t>(4 * h->sm_count, (h->n_fluid + 255) / 256 + 1);
-    rc = rc ? rc : dev_alloc(h, &h->d_red, sizeof(double) * 8 * h->red_blocks, "reduction partials");
-    rc = rc ? rc : dev_alloc(h, &h->d_red_out, sizeof(double) * 8, "reduction result");
+    // one allocation for all of them (each cudaMalloc takes longer than a small
+    // lattice's index); the first three are cleared
+    struct Want {
+        void** p;
+        size_t bytes;
+    };
+    std::vector<Want> want = {{&h->d_f[0], h->elem * 19 * h->np},
+                              {&h->d_f[1], h->elem * 19 * h->np},
+                              {&h->d_vprev, rbytes * 3 * h->np},
+                              {&h->d_rho, rbytes * h->np},
+                              {&h->d_v, rbytes * 3 * h->np},
+                              {(void**)&h->d_red, sizeof(double) * 8 * h->red_blocks},
+                              {(void**)&h->d_red_out, sizeof(double) * 8}};
+    if (h->p.two_phase) {
+        want.push_back({&h->d_psi, rbytes * h->np});
+        want.push_back({(void**)&h->d_psi0, sizeof(float) * h->ncell});
+        want.push_back({&h->d_rr, rbytes * h->np});
+        want.push_back({&h->d_rb, rbytes * h->np});
+        want.push_back({&h->d_crec, rbytes * 4 * h->np});
+        want.push_back({&h->d_pull_vz, rbytes * h->np});
+        want.push_back({&h->d_cs, rbytes * 9 * h->np});
+    }
+    size_t total = 0, clear = 0;
+    for (size_t q = 0; q < want.size(); ++q) {
+        total += (want[q].bytes + 255) / 256 * 256;
+        if (q == 2) clear = total;
+    }
+    rc = dev_alloc(h, &h->d_arena, total, "lattice arrays");
     if (rc) { free_lattice(h); return rc; }
-    rc = lbm_cuda_check(h, cudaMemsetAsync(h->d_f[0], 0, h->elem * 19 * h->np, h->stream), "clear f");
-    if (!rc) rc = lbm_cuda_check(h, cudaMemsetAsync(h->d_f[1], 0, h->elem * 19 * h->np, h->stream), "clear f");
-    if (!rc) rc = lbm_cuda_check(h, cudaMemsetAsync(h->d_vprev, 0, rbytes * 3 * h->np, h->stream), "clear vprev");
+    size_t at = 0;
+    for (const Want& w : want) {
+        *w.p = (char*)h->d_arena + at;
+        at += (w.bytes + 255) / 256 * 256;
+    }
+    rc = lbm_cuda_check(h, cudaMemsetAsync(h->d_arena, 0, clear, h->stream), "clear f, vprev");
     if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "lbm_set_geometry");
     if (rc) { free_lattice(h); return rc; }
     h->have_geometry = true;
@@ -524,12 +530,14 @@ int lbm_get_stream(LbmHandle* h, void** stream) {
 }  // extern "C"
 
 namespace {
-// Copy a node-ordered device array (n components of stride np, FP32 or FP64)
-// into a dense host array with `comps` interleaved components; solid cells get
-// `fill` (scattered on the device, lbm_geom.cu).
+// rho and v (either may be null) of the last step as dense host arrays.
 template <typename O>
-int scatter_dense(LbmHandle* h, const void* dsrc, int comps, O* out, O fill) {
-    return geom_dense_out<O>(h, dsrc, comps, out, fill);
+int macros_dense(LbmHandle* h, O* rho, O* v) {
+    GeomDense<O> want[2];
+    int n = 0;
+    if (rho) want[n++] = {h->d_rho, 1, rho, (O)1, nullptr};
+    if (v) want[n++] = {h->d_v, 3, v, (O)0, nullptr};
+    return n ? geom_dense_out<O>(h, want, n) : LBM_OK;
 }
 }  // namespace
 
@@ -546,10 +554,7 @@ int lbm_get_macros(LbmHandle* h, float* rho, float* v) {
         if (v) for (int64_t c = 0; c < 3 * h->ncell; ++c) v[c] = 0.0f;
         return LBM_OK;
     }
-    int rc = LBM_OK;
-    if (rho) rc = scatter_dense<float>(h, h->d_rho, 1, rho, 1.0f);
-    if (!rc && v) rc = scatter_dense<float>(h, h->d_v, 3, v, 0.0f);
-    return rc;
+    return macros_dense<float>(h, rho, v);
 }
 
 int lbm_get_macros_f64(LbmHandle* h, double* rho, double* v) {
@@ -561,10 +566,7 @@ int lbm_get_macros_f64(LbmHandle* h, double* rho, double* v) {
         if (v) for (int64_t c = 0; c < 3 * h->ncell; ++c) v[c] = 0.0;
         return LBM_OK;
     }
-    int rc = LBM_OK;
-    if (rho) rc = scatter_dense<double>(h, h->d_rho, 1, rho, 1.0);
-    if (!rc && v) rc = scatter_dense<double>(h, h->d_v, 3, v, 0.0);
-    return rc;
+    return macros_dense<double>(h, rho, v);
 }
 
 int lbm_get_psi(LbmHandle* h, float* psi) {
@@ -577,14 +579,13 @@ int lbm_get_phase(LbmHandle* h, float* psi, float* rho_r, float* rho_b) {
     if (!h->p.two_phase) return lbm_set_err(h, LBM_ESTATE, "lbm_get_phase: handle is single phase");
     if (!h->initialized) return lbm_set_err(h, LBM_ESTATE, "lbm_get_phase: call lbm_init first");
     cudaSetDevice(h->device);
-    int rc = LBM_OK;
-    if (psi) {
-        // solid cells keep the input psi (the reference never updates them)
-        rc = geom_dense_out<float>(h, h->d_psi, 1, psi, 0.0f, h->d_psi0);
-    }
-    if (!rc && rho_r) rc = scatter_dense<float>(h, h->d_rr, 1, rho_r, 0.0f);
-    if (!rc && rho_b) rc = scatter_dense<float>(h, h->d_rb, 1, rho_b, 0.0f);
-    return rc;
+    GeomDense<float> want[3];
+    int n = 0;
+    // solid cells keep the input psi (the reference never updates them)
+    if (psi) want[n++] = {h->d_psi, 1, psi, 0.0f, h->d_psi0};
+    if (rho_r) want[n++] = {h->d_rr, 1, rho_r, 0.0f, nullptr};
+    if (rho_b) want[n++] = {h->d_rb, 1, rho_b, 0.0f, nullptr};
+    return n ? geom_dense_out<float>(h, want, n) : LBM_OK;
 }
 
 int lbm_reductions(LbmHandle* h, LbmStats* out) {

@@ -81,6 +81,7 @@ struct LbmHandle {
     uint32_t* d_coord = nullptr;           // packed (i,j,k) per node
     void* d_links = nullptr;               // neighbour links (lbm_links.cuh), one allocation
     LbmLinks links{};
+    void* d_arena = nullptr;               // one allocation holding the arrays below (grey's aside)
     void* d_f[2] = {nullptr, nullptr};     // populations, 19 x np elements in AoSoA-32 chunks
     int cur = 0;
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};   // a run of steps from each buffer order (lbm_capi.cu)
@@ -115,8 +116,21 @@ int geom_build(LbmHandle* h, const int8_t* solid, int64_t si, int64_t sj, int64_
 int geom_host_index(LbmHandle* h);
 // Neighbour links (lbm_links.cu).
 int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count);
+// A node-ordered device array (comps components of stride np, the handle's
+// compute type) wanted as a dense host array: comps interleaved per cell, solid
+// cells `fill`, or fill_cells[c] where given.
 template <typename O>
-int geom_dense_out(LbmHandle* h, const void* dsrc, int comps, O* out, O fill, const O* fill_cells = nullptr);
+struct GeomDense {
+    const void* src;
+    int comps;
+    O* out;
+    O fill;
+    const O* fill_cells;
+};
+template <typename O>
+int geom_dense_out(LbmHandle* h, const GeomDense<O>* want, int count);
+// Touch every page of a host range about to be filled, in parallel.
+void host_touch(void* const* p, const size_t* bytes, int count);
 
 // single phase (lbm_sp.cu)
 int sp_launch_init(LbmHandle* h, const void* rho_nodes, const void* v_nodes);

@@ -28,10 +28,11 @@
 // only when the caller reads them next (MACROS) or, for v, where a pressure
 // face needs the previous step's.
 //
-// 131^3 drainage, FP32, 894k nodes: 82.7 us a step against 98.4 with six scalar
+// 131^3 drainage, FP32, 894k nodes: 81.8 us a step against 98.4 with six scalar
 // loads a direction and map lookups.  Launch A is bound by L1 wavefronts (every
 // direction reads its own 24 unaligned bytes: 68% of the data pipe), launch B by
-// issue slots and latency at 64 registers.  Storing the 38 recoloured
+// issue slots and latency; its psi loads wait together with the
+// populations' (after the faces 83.0 us).  Storing the 38 recoloured
 // populations instead (two values a direction in launch A) took a third of the
 // wavefronts but 140 MB more DRAM traffic a step: 94 us.
 #include <cuda_runtime.h>
@@ -42,12 +43,13 @@
 #include "lbm_linkgather.cuh"
 
 // Resident 128-thread CTAs per SM of the two launches (FP32 and 16-bit), us a step
-// on the same lattice: 10 and 8 82.7; 9 and 7 88.1; 12 and 7 84.2; 11 and 6 86.9.
+// on the same lattice / on a 50 x 44 x 37 sample: 10 and 7 81.8 / 13.3; 10 and 8
+// 81.7 / 14.6; 10 and 9 86.6 / 16.4; 10 and 6 87.5 / 15.6; 9 and 7 88.1, 12 and 7 84.2.
 #ifndef LBM_TP_MINBLOCKS_A
 #define LBM_TP_MINBLOCKS_A 10
 #endif
 #ifndef LBM_TP_MINBLOCKS_B
-#define LBM_TP_MINBLOCKS_B 8
+#define LBM_TP_MINBLOCKS_B 7
 #endif
 
 namespace {
@@ -424,6 +426,11 @@ __global__ void __launch_bounds__(128, STORE == LBM_STORE_F64 ? 2 : LBM_TP_MINBL
     const R rr = launder(rr_new)[n], rb = launder(rb_new)[n];
     R F[19];
     LinkGather<STORE, Cd::RHOREF>::all(F, fin, L, K, n, rx);
+    // (before the faces: its loads then wait together with those of F)
+    R Cx, Cy, Cz;
+    if (K.bits & (LBM_LINK_EDGE | LBM_LINK_EXC)) colour_gradient<R>(T, map, psi, i, j, k, rr, rb, Cx, Cy, Cz);
+    else colour_gradient_links<R>(T, K, n, psi, rr, rb, Cx, Cy, Cz);
+    const R psi_own = psi[n];
     if (K.bits & LBM_LINK_FACE) apply_faces<R, Cd::DEV>(F, i, j, k, n, C, map, v);  // v: previous step
     R r = F[0];
 #pragma unroll
@@ -437,10 +444,7 @@ __global__ void __launch_bounds__(128, STORE == LBM_STORE_F64 ? 2 : LBM_TP_MINBL
         v[np + n] = vy;
         v[2 * np + n] = vz;
     }
-    R Cx, Cy, Cz;
-    if (K.bits & (LBM_LINK_EDGE | LBM_LINK_EXC)) colour_gradient<R>(T, map, psi, i, j, k, rr, rb, Cx, Cy, Cz);
-    else colour_gradient_links<R>(T, K, n, psi, rr, rb, Cx, Cy, Cz);
-    tp_collide_and_store<STORE, FORCE>(F, r, vx, vy, vz, n, rx.at, T, Cx, Cy, Cz, psi[n], rr, rb, fout, crec,
+    tp_collide_and_store<STORE, FORCE>(F, r, vx, vy, vz, n, rx.at, T, Cx, Cy, Cz, psi_own, rr, rb, fout, crec,
                                        pull_vz, cs_out);
 }
 

@@ -658,8 +658,9 @@ __global__ void __launch_bounds__(TMA_THREADS) conv3d_halo_kernel(const HaloArgs
 }
 
 // ---------------------------------------------------------------------------
-// Warp-specialised weight gradient for layers whose input and output are one
-// channel part each (16, 32 or 64 channels): the same GEMM, tap groups, ones
+// Warp-specialised weight gradient for layers whose output is one channel part
+// (16, 32 or 64 channels) and whose input is one, or three of 16 (a CTA per
+// part, blockIdx.y): the same GEMM, tap groups, ones
 // slot and partials as conv3d_wgrad_tma_kernel, but each 8 x 4 x 4 block is
 // loaded once -- one dense TMA box of the 10 x 6 x 6 input halo and one of g
 // (no swizzle) -- and a CTA runs all tap groups of its blocks, one TMEM
@@ -679,7 +680,8 @@ constexpr int WS_THREADS = 160;
 struct WsArgs {
     CUtensorMap halo;               // input, tiled 5-D (cin, W, H, D, N), box (cin, 10, 6, 6, 1), no swizzle
     CUtensorMap gmap;               // g, tiled 5-D (cout, W, H, D, N), box (cout, 8, 4, 4, 1), no swizzle
-    int cin, cout, tg, ngroups;     // tap slots per group (128 / cin), groups (ceil(27 / tg))
+    int cin, cout, tg, ngroups;     // channels of a part, tap slots per group (128 / cin), groups (ceil(27 / tg))
+    int cin_all;                    // channels of the input: cin_all / cin parts, one per blockIdx.y
     uint32_t hbytes;                // bytes of the halo box
     uint32_t tbytes;                // bytes of one TMA buffer (halo then g), 1024-aligned
     uint32_t obytes;                // bytes of one operand buffer (32 KB of tap slots + g), 1024-aligned
@@ -705,6 +707,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
     const int64_t chunk = blockIdx.x;
     const int64_t b0 = chunk * P.chunk_blocks;
     const int nb = (int)min((int64_t)P.chunk_blocks, P.nblocks - b0);
+    const int part0 = (int)blockIdx.y * P.cin;           // first input channel of the part (a multiple of 16)
     const int pw = P.cin, tg = P.tg, ng = P.ngroups;
     const uint32_t span = 2u * (uint32_t)pw;
     const uint32_t gs = 2u * (uint32_t)COUT;
@@ -751,7 +754,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
                 asm volatile(
                     "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
                     " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(tb),
-                    "l"(&P.halo), "r"(0), "r"(w0 - 1), "r"(h0 - 1), "r"(d0 - 1), "r"(n), "r"(bar)
+                    "l"(&P.halo), "r"(part0), "r"(w0 - 1), "r"(h0 - 1), "r"(d0 - 1), "r"(n), "r"(bar)
                     : "memory");
                 asm volatile(
                     "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
@@ -866,10 +869,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
                 float acc[16];
                 tmem_ld16(tw + (uint32_t)(gi * COUT + c0), acc);
                 if (sl < ntap) {
-                    float* dst = part + ((chunk * 27 + gi * tg + sl) * COUT + c0) * P.cin + cil;
+                    float* dst = part + ((chunk * 27 + gi * tg + sl) * COUT + c0) * P.cin_all + part0 + cil;
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) dst[(int64_t)q * P.cin] = acc[q];
-                } else if (gi == ng - 1 && sl == ntap && cil == 0) {
+                    for (int q = 0; q < 16; ++q) dst[(int64_t)q * P.cin_all] = acc[q];
+                } else if (gi == ng - 1 && sl == ntap && cil == 0 && part0 == 0) {
 #pragma unroll
                     for (int q = 0; q < 16; ++q) dbpart[chunk * COUT + c0 + q] = acc[q];
                 }
@@ -1198,8 +1201,12 @@ int nn_wgrad_tma(const void* in, const void* g, float* part, float* dbpart, int 
 // two CTAs fit an SM (113 KB) or cout = 64 > cin: with one CTA per SM the
 // TMA-box kernel was faster on 16 -> 32 and 32 -> 32 (2 x 48^3), while on 32 -> 64
 // the per-group reload of the 64-channel g made that kernel the slower one.
-// LBM_NN_WS=0 in the environment turns it off.
-static bool ws_plan(int cin, int cout, WsArgs* P, size_t* smem) {
+// 48 -> 16 runs as three parts of 16 channels: 870 us on 2 x 96^3 (partial
+// reduction included) against 1114 with the TMA-box kernel (48 channels in one
+// part need 1598: one CTA per SM).  LBM_NN_WS=0 in the environment turns it off.
+static bool ws_plan(int cin_all, int cout, WsArgs* P, size_t* smem) {
+    const int cin = cin_all == 48 && cout == 16 ? 16 : cin_all;   // channels of a part
+    P->cin_all = cin_all;
     if (!(cin == 16 || cin == 32 || cin == 64) || !(cout == 16 || cout == 32 || cout == 64)) return false;
     P->cin = cin;
     P->cout = cout;
@@ -1256,7 +1263,7 @@ int nn_wgrad_ws(const void* in, const void* g, float* part, float* dbpart, int n
         const cuuint64_t dim[5] = {(cuuint64_t)cin, (cuuint64_t)wd, (cuuint64_t)h, (cuuint64_t)d, (cuuint64_t)n};
         const cuuint64_t str[4] = {(cuuint64_t)cin * 2, (cuuint64_t)wd * cin * 2, (cuuint64_t)h * wd * cin * 2,
                                    (cuuint64_t)d * h * wd * cin * 2};
-        const cuuint32_t box[5] = {(cuuint32_t)cin, 10, 6, 6, 1};
+        const cuuint32_t box[5] = {(cuuint32_t)P.cin, 10, 6, 6, 1};
         const CUresult r = g_enc_tiled(&P.halo, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(in), dim, str, box,
                                        es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1281,7 +1288,7 @@ int nn_wgrad_ws(const void* in, const void* g, float* part, float* dbpart, int n
         auto k = conv3d_wgrad_ws_kernel<C>;                                                                      \
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)      \
             return lbm_set_err(nullptr, LBM_ECUDA, "lbm_nn_conv3d_wgrad (ws): shared memory attribute refused"); \
-        k<<<(unsigned)nchunk, WS_THREADS, smem, s>>>(P, part, dbpart);                                           \
+        k<<<dim3((unsigned)nchunk, (unsigned)(cin / P.cin)), WS_THREADS, smem, s>>>(P, part, dbpart);            \
         break;                                                                                                   \
     }
     switch (cout) {

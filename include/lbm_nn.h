@@ -94,6 +94,23 @@ int lbm_nn_mse(const float* y, const float* t, const uint8_t* mask, float* gy, f
 int lbm_nn_adam(float* p, const float* g, float* m, float* v, void* p16, int64_t n, float lr, float b1, float b2,
                 float eps, int32_t step, float weight_decay, void* stream);
 
+/* The same step over several tensors in one launch.  A conv weight ([cout][27][cin],
+ * n = 27 cin cout) also gets its BF16 copy w16 and the flip-transposed wt16
+ * (lbm_nn_flip_transpose of w16); both are NULL for the others. */
+#define LBM_NN_ADAM_MAX 32
+typedef struct LbmNnAdamTensor {
+    float* p;
+    const float* g;
+    float* m;
+    float* v;
+    void* w16;
+    void* wt16;
+    int64_t n;
+    int32_t cin, cout;
+} LbmNnAdamTensor;
+int lbm_nn_adam_many(const LbmNnAdamTensor* t, int32_t count, float lr, float b1, float b2, float eps, int32_t step,
+                     float weight_decay, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -49,7 +49,12 @@ _SIGS = {
     "lbm_nn_head_bwd": ([_P, _P, _P, _P, _P, _P, _L, _I, _I, _P], ctypes.c_int),
     "lbm_nn_mse": ([_P, _P, _P, _P, _P, _P, _L, _I, _F, _P], ctypes.c_int),
     "lbm_nn_adam": ([_P, _P, _P, _P, _P, _L, _F, _F, _F, _F, _I, _F, _P], ctypes.c_int),
+    "lbm_nn_adam_many": ([_P, _I, _F, _F, _F, _F, _I, _F, _P], ctypes.c_int),
 }
+
+
+class _AdamTensor(ctypes.Structure):
+    _fields_ = [(k, _P) for k in ("p", "g", "m", "v", "w16", "wt16")] + [("n", _L), ("cin", _I), ("cout", _I)]
 
 
 def _lib():
@@ -328,16 +333,22 @@ class UNet3D:
         s = self._stream()
         self.step_count += 1
         hw_hb_g = self.ghw_hb
-        items = [(self.w[k], self.gw[k], None) for k in self.w] + [(self.b[k], self.gb[k], None) for k in self.b]
+        # (master, gradient, layer of a conv weight or None): one launch updates all of
+        # them and the BF16 copies that the next step's convolutions read
+        items = [(self.w[k], self.gw[k], k) for k in self.w] + [(self.b[k], self.gb[k], None) for k in self.b]
         items += [(self.hw, hw_hb_g[:OUT * 16].view(OUT, 16), None), (self.hb, hw_hb_g[OUT * 16:], None)]
-        for p, g, _ in items:
+        shape = {name: (cin, cout) for name, cin, cout, _ in LAYERS}
+        rows = (_AdamTensor * len(items))()
+        for r, (p, g, name) in zip(rows, items):
             key = p.data_ptr()
             if key not in self.adam:
                 self.adam[key] = (self.torch.zeros_like(p), self.torch.zeros_like(p))
             m, v = self.adam[key]
-            _ck(L.lbm_nn_adam(_p(p), _p(g.contiguous()), _p(m), _p(v), None, p.numel(), lr, b1, b2, eps,
-                              self.step_count, weight_decay, s))
-        self.refresh()
+            r.p, r.g, r.m, r.v, r.n = key, g.data_ptr(), m.data_ptr(), v.data_ptr(), p.numel()
+            if name is not None:
+                r.w16, r.wt16 = self.w16[name].data_ptr(), self.wt16[name].data_ptr()
+                r.cin, r.cout = shape[name]
+        _ck(L.lbm_nn_adam_many(ctypes.addressof(rows), len(items), lr, b1, b2, eps, self.step_count, weight_decay, s))
 
 
 def features(solid):

@@ -153,3 +153,51 @@ def test_head_weight_gradient_one_pass_matches_fp64_and_general_form():
     for o in out:
         assert np.abs(o - ref).max() / np.abs(ref).max() < 1e-5
     assert np.abs(out[0] - out[1]).max() / np.abs(ref).max() < 1e-5
+
+
+@pytest.mark.parametrize("nvox", [1, 255, 256, 257, 4801])
+@pytest.mark.parametrize("act", [0, 1])
+def test_head_vector_equals_elementwise(nvox, act):
+    """The 16 -> 4 head, forward and backward data: aligned tensors (whole vectors) against shifted ones."""
+    import torch
+    L = _lib()
+    torch.manual_seed(nvox)
+    x = torch.randn(nvox, 16)
+    xa, xu = _pair(x if act else x.relu(), (nvox, 16), torch.bfloat16)
+    w, b = torch.randn(4, 16).cuda(), torch.randn(4).cuda()
+    ya, yu = _pair(torch.zeros(nvox, 4), (nvox, 4), torch.float32)
+    assert L.lbm_nn_head(_p(xa), _p(w), _p(b), _p(ya), nvox, 16, 4, _s()) == 0
+    assert L.lbm_nn_head(_p(xu), _p(w), _p(b), _p(yu), nvox, 16, 4, _s()) == 0
+    _same(ya, yu)
+    gy = torch.randn(nvox, 4).cuda()
+    ga, gu = _pair(torch.zeros(nvox, 16), (nvox, 16), torch.bfloat16)
+    scr, dwdb = torch.empty(256 * 68, device="cuda"), torch.empty(68, device="cuda")
+    for xx, gx in ((xa, ga), (xu, gu)):
+        assert L.lbm_nn_head_bwd_act(_p(gy), _p(w), _p(xx), _p(xx), _p(gx), _p(dwdb), _p(scr), nvox, 16, 4, act,
+                                     _s()) == 0
+    _same(ga, gu)
+
+
+def test_adam_many_equals_single_tensor_steps_and_refresh():
+    import torch
+    from taichi_lbm3d_gb300.unet import UNet3D
+    L = _lib()
+    m = UNet3D(seed=3)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for t in list(m.gw.values()) + list(m.gb.values()) + [m.ghw_hb]:
+        t.copy_(torch.randn(t.shape, generator=g, device="cuda") * 1e-2)
+    params = [(k, p, q) for k, p, q in [(k, m.w[k], m.gw[k]) for k in m.w] + [(None, m.b[k], m.gb[k]) for k in m.b]
+              + [(None, m.hw, m.ghw_hb[:64].view(4, 16)), (None, m.hb, m.ghw_hb[64:])]]
+    ref = [(p.clone(), torch.zeros_like(p), torch.zeros_like(p)) for _, p, _ in params]
+    for step in (1, 2, 3):
+        m.adam_step(lr=1e-3, weight_decay=1e-2)
+        for (_, _, q), (p, mm, vv) in zip(params, ref):
+            assert L.lbm_nn_adam(_p(p), _p(q), _p(mm), _p(vv), None, p.numel(), 1e-3, 0.9, 0.999, 1e-8, step, 1e-2,
+                                 _s()) == 0
+    for (_, p, _), (r, _, _) in zip(params, ref):
+        _same(p, r)
+    w16, wt16 = {k: v.clone() for k, v in m.w16.items()}, {k: v.clone() for k, v in m.wt16.items()}
+    m.refresh()
+    for k in m.w16:
+        _same(w16[k], m.w16[k])
+        _same(wt16[k], m.wt16[k])

@@ -70,6 +70,14 @@ int lbm_nn_upsample2_bwd(const void* gout, void* gin, const void* mask, int32_t 
 int lbm_nn_concat(const void* a, int32_t ca, const void* b, int32_t cb, void* out, int64_t nvox, void* stream);
 int lbm_nn_split(const void* g, int32_t ca, int32_t cb, void* ga, void* gb, const void* mask_b, int32_t accumulate_b,
                  int64_t nvox, void* stream);
+/* The decoder's upsample2 of low (ca channels, dims n, d, h, w) concatenated with
+ * skip (cb channels, twice the dims) in one pass, and its gradient: glow as
+ * lbm_nn_upsample2_bwd of g[:, :ca] with mask, gskip = g[:, ca:].  Channels are
+ * multiples of 8, tensors 16-byte aligned. */
+int lbm_nn_upcat(const void* low, int32_t ca, const void* skip, int32_t cb, void* out, int32_t n, int32_t d, int32_t h,
+                 int32_t w, void* stream);
+int lbm_nn_upcat_bwd(const void* g, int32_t ca, int32_t cb, void* glow, const void* mask, void* gskip, int32_t n, int32_t d,
+                     int32_t h, int32_t w, void* stream);
 /* 1x1 output head y = x w^T + b (FP32 out; cin <= 64, cout <= 8), and its
  * backward: gx = (x > 0) * gy w; dw_db = [dw (cout*cin) | db (cout)];
  * scratch of 256 * (cout*cin + cout) floats. */

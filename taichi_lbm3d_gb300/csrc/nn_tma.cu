@@ -659,23 +659,30 @@ __global__ void __launch_bounds__(TMA_THREADS) conv3d_halo_kernel(const HaloArgs
 
 // ---------------------------------------------------------------------------
 // Warp-specialised weight gradient for layers whose output is one channel part
-// (16, 32 or 64 channels) and whose input is one, or three of 16 (a CTA per
+// (16, 32 or 64 channels) and whose input is one, or several of 16 (a CTA per
 // part, blockIdx.y): the same GEMM, tap groups, ones
 // slot and partials as conv3d_wgrad_tma_kernel, but each 8 x 4 x 4 block is
 // loaded once -- one dense TMA box of the 10 x 6 x 6 input halo and one of g
 // (no swizzle) -- and a CTA runs all tap groups of its blocks, one TMEM
 // accumulator per group.
-//   warp 4, lane 0: TMA producer (two boxes per block, two buffers) and MMA
+//   last warp, lane 0: TMA producer (two boxes per block, two buffers) and MMA
 //     issuer (8 K = 16 steps per block and group, two operand buffers);
-//   warps 0-3: build the operand buffer of each (block, group) step from the
+//   warps 0-7: build the operand buffer of each (block, group) step from the
 //     halo -- tap slot j row r is the halo voxel r shifted by the tap, written
-//     in the swizzled MN-major layout -- plus the g operand, then the epilogue.
+//     in the swizzled MN-major layout -- and once per block the g operand
+//     (its own two buffers); warps 0-3 run the epilogue.
 // mbarriers between the roles: tfull (TMA -> copy), tempty (copy -> producer,
-// 128 arrivals), ofull (copy -> MMA, 128 arrivals), oempty (MMA commit ->
+// WS_COPY arrivals), ofull (copy -> MMA, WS_COPY arrivals), oempty (MMA commit ->
 // copy), done.  Every wait is bounded; a timeout records the error flag and
 // the roles leave their loops, the producer first waiting (bounded) for the
 // loads it issued.
-constexpr int WS_THREADS = 160;
+// The copies bound it: 64 KB through shared memory a step.  Copy warps and g, us
+// with the partial reduction on 2 x 96^3, 16 -> 16 / 48 -> 16: 4 warps, g with every
+// step 310 / 870; 4 warps, g once a block 299 / 849; 8 warps 230 / 624; 16 warps
+// 397 / 1099 (one CTA per SM).
+constexpr int WS_COPY = 256;                     // threads that build operands
+constexpr int WS_THREADS = WS_COPY + 32;
+constexpr int WS_CHUNKS = 2048 / WS_COPY;        // 16-byte pieces of a step's tap slots per thread
 
 struct WsArgs {
     CUtensorMap halo;               // input, tiled 5-D (cin, W, H, D, N), box (cin, 10, 6, 6, 1), no swizzle
@@ -684,7 +691,8 @@ struct WsArgs {
     int cin_all;                    // channels of the input: cin_all / cin parts, one per blockIdx.y
     uint32_t hbytes;                // bytes of the halo box
     uint32_t tbytes;                // bytes of one TMA buffer (halo then g), 1024-aligned
-    uint32_t obytes;                // bytes of one operand buffer (32 KB of tap slots + g), 1024-aligned
+    uint32_t obytes;                // bytes of one operand buffer (32 KB of tap slots)
+    uint32_t gbytes;                // bytes of one g operand buffer, 1024-aligned
     uint32_t ncol;                  // TMEM columns (power of two >= ngroups x cout)
     int shift[27];                  // byte offset of tap t's shift inside the halo
     int nbw, nbh, nbd;
@@ -704,6 +712,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t base = (su32(dsmem) + 1023u) & ~1023u;
     const uint32_t obase = base + 2u * P.tbytes;
+    const uint32_t gbase = obase + 2u * P.obytes;
     const int64_t chunk = blockIdx.x;
     const int64_t b0 = chunk * P.chunk_blocks;
     const int nb = (int)min((int64_t)P.chunk_blocks, P.nblocks - b0);
@@ -716,8 +725,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&s_tfull[b])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(su32(&s_tempty[b])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 128;" ::"r"(su32(&s_ofull[b])) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(&s_tempty[b])), "n"(WS_COPY) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(su32(&s_ofull[b])), "n"(WS_COPY) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&s_oempty[b])) : "memory");
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(su32(&s_done)) : "memory");
@@ -736,7 +745,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
     const uint32_t taddr = s_taddr;
     const int nsteps = nb * ng;
 
-    if (warp == 4) {
+    if (warp == WS_COPY / 32) {
         if ((tid & 31) == 0) {   // producer + MMA issuer
             const uint32_t tx = P.hbytes + 128u * gs;
             auto issue = [&](int b) {
@@ -771,12 +780,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
                 if (gi == 0) landed = b + 1;   // the copy warps saw block b's loads complete
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t sa = obase + (uint32_t)ob * P.obytes;
+                const uint32_t gb = gbase + (uint32_t)(b & 1) * P.gbytes;
                 const uint32_t acc = taddr + (uint32_t)(gi * COUT);
 #pragma unroll 1
                 for (int kk = 0; kk < 8; ++kk) {
                     const uint64_t ad = mn_desc(sa + (uint32_t)kk * 16u * span, 128u * span, 8u * span, (int)span);
                     const uint64_t bdsc =
-                        mn_desc(sa + 32768u + (uint32_t)kk * 16u * gs, 8u * gs, 8u * gs, (int)gs);
+                        mn_desc(gb + (uint32_t)kk * 16u * gs, 8u * gs, 8u * gs, (int)gs);
                     mma_f16(acc, ad, bdsc, idesc_mn(128, COUT), (b | kk) != 0 ? 1u : 0u);
                 }
                 mma_commit(&s_oempty[ob]);
@@ -797,10 +807,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
         // copy warps: the per-thread chunks of a step are fixed; tap t adds P.shift[t] to the source
         const int csh = pw == 64 ? 3 : (pw == 32 ? 2 : 1);
         // packed: source offset in the halo (< 46 KB) | destination offset in the tap slots (< 32 KB) << 16
-        uint32_t pk[16];
+        uint32_t pk[WS_CHUNKS];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-            const int e = tid + k * 128;
+        for (int k = 0; k < WS_CHUNKS; ++k) {
+            const int e = tid + k * WS_COPY;
             const int c = e & ((1 << csh) - 1);
             const int r = (e >> csh) & 127;
             const int j = e >> (7 + csh);                     // tap slot (< tg)
@@ -819,8 +829,8 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
             const uint32_t osh = obase + (uint32_t)ob * P.obytes;
             const int ntap = gi == ng - 1 ? ntap_last : tg;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) {
-                const int j = (tid + k * 128) >> (7 + csh);
+            for (int k = 0; k < WS_CHUNKS; ++k) {
+                const int j = (tid + k * WS_COPY) >> (7 + csh);
                 if (j < ntap) {
                     uint32_t v0, v1, v2, v3;
                     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
@@ -834,13 +844,15 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
                     asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(osh + (pk[k] >> 16)), "r"(one) : "memory");
                 }
             }
-            for (int e = tid; e < 128 * gch; e += 128) {        // g operand: row r, chunk c8
+            // g operand, once a block (the block two before no longer reads this buffer:
+            // the wait above saw all but its successor's last steps done): row r, chunk c8
+            for (int e = gi == 0 ? tid : 128 * gch; e < 128 * gch; e += WS_COPY) {
                 const int c8 = e % gch, r = e / gch;
                 uint32_t v0, v1, v2, v3;
                 asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                              : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
                              : "r"(tsh + P.hbytes + (uint32_t)r * gs + (uint32_t)c8 * 16u));
-                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(osh + 32768u + swz((uint32_t)r, (uint32_t)c8, gs)),
+                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(gbase + (uint32_t)(b & 1) * P.gbytes + swz((uint32_t)r, (uint32_t)c8, gs)),
                              "r"(v0), "r"(v1), "r"(v2), "r"(v3)
                              : "memory");
             }
@@ -1198,14 +1210,16 @@ int nn_wgrad_tma(const void* in, const void* g, float* part, float* dbpart, int 
 
 // Warp-specialised weight gradient: one-part layers (cin and cout in {16, 32, 64})
 // whose accumulators (groups x cout columns) and buffers fit.  It is taken where
-// two CTAs fit an SM (113 KB) or cout = 64 > cin: with one CTA per SM the
+// two CTAs fit an SM (113 KB) or cout = 64: with one CTA per SM the
 // TMA-box kernel was faster on 16 -> 32 and 32 -> 32 (2 x 48^3), while on 32 -> 64
 // the per-group reload of the 64-channel g made that kernel the slower one.
-// 48 -> 16 runs as three parts of 16 channels: 870 us on 2 x 96^3 (partial
+// 64 -> 64 runs as four parts of 16 channels (2 x 24^3: 55 us against 77), 48 -> 16
+// as three: 624 us on 2 x 96^3 (partial
 // reduction included) against 1114 with the TMA-box kernel (48 channels in one
 // part need 1598: one CTA per SM).  LBM_NN_WS=0 in the environment turns it off.
 static bool ws_plan(int cin_all, int cout, WsArgs* P, size_t* smem) {
-    const int cin = cin_all == 48 && cout == 16 ? 16 : cin_all;   // channels of a part
+    // channels of a part
+    const int cin = (cin_all == 48 && cout == 16) || (cin_all == 64 && cout == 64) ? 16 : cin_all;
     P->cin_all = cin_all;
     if (!(cin == 16 || cin == 32 || cin == 64) || !(cout == 16 || cout == 32 || cout == 64)) return false;
     P->cin = cin;
@@ -1217,9 +1231,10 @@ static bool ws_plan(int cin_all, int cout, WsArgs* P, size_t* smem) {
     while (P->ncol < (uint32_t)(P->ngroups * cout)) P->ncol <<= 1;
     P->hbytes = 360u * (uint32_t)cin * 2u;
     P->tbytes = (P->hbytes + 128u * 2u * (uint32_t)cout + 1023u) & ~1023u;
-    P->obytes = 32768u + ((128u * 2u * (uint32_t)cout + 1023u) & ~1023u);
+    P->obytes = 32768u;
+    P->gbytes = (128u * 2u * (uint32_t)cout + 1023u) & ~1023u;
     for (int t = 0; t < 27; ++t) P->shift[t] = ((t / 9) * 60 + ((t / 3) % 3) * 10 + t % 3) * cin * 2;
-    *smem = 2 * (size_t)P->tbytes + 2 * (size_t)P->obytes + 1024;
+    *smem = 2 * ((size_t)P->tbytes + P->obytes + P->gbytes) + 1024;
     return *smem <= 227 * 1024;
 }
 
@@ -1243,7 +1258,7 @@ bool nn_wgrad_ws_usable(int cin, int cout) {
     WsArgs P{};
     size_t smem = 0;
     if (!on || !encoders() || !ws_plan(cin, cout, &P, &smem)) return false;
-    return smem <= 113 * 1024 || (cout == 64 && cin < cout);
+    return smem <= 113 * 1024 || cout == 64;
 }
 
 // Partials for nn_wgrad_ws_chunks(n, d, h, w) chunks of the same 8 x 4 x 4 blocks.

@@ -45,6 +45,8 @@ _SIGS = {
     "lbm_nn_upsample2_bwd": ([_P, _P, _P, _I, _I, _I, _I, _I, _P], ctypes.c_int),
     "lbm_nn_concat": ([_P, _I, _P, _I, _P, _L, _P], ctypes.c_int),
     "lbm_nn_split": ([_P, _I, _I, _P, _P, _P, _I, _L, _P], ctypes.c_int),
+    "lbm_nn_upcat": ([_P, _I, _P, _I, _P, _I, _I, _I, _I, _P], ctypes.c_int),
+    "lbm_nn_upcat_bwd": ([_P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _P], ctypes.c_int),
     "lbm_nn_head": ([_P, _P, _P, _P, _L, _I, _I, _P], ctypes.c_int),
     "lbm_nn_head_bwd": ([_P, _P, _P, _P, _P, _P, _L, _I, _I, _P], ctypes.c_int),
     "lbm_nn_mse": ([_P, _P, _P, _P, _P, _P, _L, _I, _F, _P], ctypes.c_int),
@@ -188,11 +190,8 @@ class UNet3D:
             return out
 
         def up_cat(name, src, lv_low, c, skip, cs):
-            up = self._buf("up_" + name, dims[lv_low - 1] + (c,), t.bfloat16)
-            _ck(L.lbm_nn_upsample2(_p(src), _p(up), *dims[lv_low], c, s))
             cat = self._buf("a_" + name, dims[lv_low - 1] + (c + cs,), t.bfloat16)
-            nv = int(np.prod(dims[lv_low - 1]))
-            _ck(L.lbm_nn_concat(_p(up), c, _p(skip), cs, _p(cat), nv, s))
+            _ck(L.lbm_nn_upcat(_p(src), c, _p(skip), cs, _p(cat), *dims[lv_low], s))
             a[name] = cat
             return cat
 
@@ -267,23 +266,18 @@ class UNet3D:
         g_d1 = bwd_data("d1b", g_d1b, dmask("d1"), "d1")
         wgrad("d1", a["c1"], g_d1)
         g_c1 = bwd_data("d1", g_d1, None, "c1")
-        g_u1 = g_buf("u1", 0, 32)
         g_e1b = g_buf("e1b", 0, 16)
-        _ck(L.lbm_nn_split(_p(g_c1), 32, 16, _p(g_u1), _p(g_e1b), None, 0, nv0, s))
         g_d2b = g_buf("d2b", 1, 32)
-        _ck(L.lbm_nn_upsample2_bwd(_p(g_u1), _p(g_d2b), None if gelu else _p(a["d2b"]), *dims[1], 32, s))
+        _ck(L.lbm_nn_upcat_bwd(_p(g_c1), 32, 16, _p(g_d2b), None if gelu else _p(a["d2b"]), _p(g_e1b), *dims[1], s))
         act_bwd(g_d2b, "d2b")
         # level 1 decoder
         wgrad("d2b", a["d2"], g_d2b)
         g_d2 = bwd_data("d2b", g_d2b, dmask("d2"), "d2")
         wgrad("d2", a["c2"], g_d2)
         g_c2 = bwd_data("d2", g_d2, None, "c2")
-        nv1 = int(np.prod(dims[1]))
-        g_u2 = g_buf("u2", 1, 64)
         g_e2b = g_buf("e2b", 1, 32)
-        _ck(L.lbm_nn_split(_p(g_c2), 64, 32, _p(g_u2), _p(g_e2b), None, 0, nv1, s))
         g_b1b = g_buf("b1b", 2, 64)
-        _ck(L.lbm_nn_upsample2_bwd(_p(g_u2), _p(g_b1b), None if gelu else _p(a["b1b"]), *dims[2], 64, s))
+        _ck(L.lbm_nn_upcat_bwd(_p(g_c2), 64, 32, _p(g_b1b), None if gelu else _p(a["b1b"]), _p(g_e2b), *dims[2], s))
         act_bwd(g_b1b, "b1b")
         # bottleneck
         wgrad("b1b", a["b1"], g_b1b)

@@ -201,3 +201,30 @@ def test_adam_many_equals_single_tensor_steps_and_refresh():
     for k in m.w16:
         _same(w16[k], m.w16[k])
         _same(wt16[k], m.wt16[k])
+
+
+@pytest.mark.parametrize("c,cs,dims", [(32, 16, (2, 3, 4, 5)), (64, 32, (1, 1, 1, 1)), (8, 24, (1, 2, 5, 3))])
+def test_upcat_equals_upsample_then_concat(c, cs, dims):
+    import torch
+    L = _lib()
+    torch.manual_seed(c)
+    n, d, h, w = dims
+    big = (n, 2 * d, 2 * h, 2 * w)
+    nv = int(np.prod(big))
+    bf = dict(dtype=torch.bfloat16, device="cuda")
+    low, skip = torch.randn(n, d, h, w, c).cuda().to(torch.bfloat16), torch.randn(*big, cs).cuda().to(torch.bfloat16)
+    up, cat, one = torch.empty(*big, c, **bf), torch.empty(*big, c + cs, **bf), torch.zeros(*big, c + cs, **bf)
+    assert L.lbm_nn_upsample2(_p(low), _p(up), n, d, h, w, c, _s()) == 0
+    assert L.lbm_nn_concat(_p(up), c, _p(skip), cs, _p(cat), nv, _s()) == 0
+    assert L.lbm_nn_upcat(_p(low), c, _p(skip), cs, _p(one), n, d, h, w, _s()) == 0
+    _same(cat, one)
+    g = torch.randn(*big, c + cs).cuda().to(torch.bfloat16)
+    for mask in (None, low):
+        gu, gs, gl = torch.empty(*big, c, **bf), torch.empty(*big, cs, **bf), torch.empty(n, d, h, w, c, **bf)
+        gl1, gs1 = torch.zeros_like(gl), torch.zeros_like(gs)
+        assert L.lbm_nn_split(_p(g), c, cs, _p(gu), _p(gs), None, 0, nv, _s()) == 0
+        assert L.lbm_nn_upsample2_bwd(_p(gu), _p(gl), _p(mask), n, d, h, w, c, _s()) == 0
+        assert L.lbm_nn_upcat_bwd(_p(g), c, cs, _p(gl1), _p(mask), _p(gs1), n, d, h, w, _s()) == 0
+        _same(gl, gl1)
+        _same(gs, gs1)
+    assert L.lbm_nn_upcat(_p(low), 12, _p(skip), cs, _p(one), n, d, h, w, _s()) != 0

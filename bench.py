@@ -613,7 +613,7 @@ def unet_layers(n=2, edge=96, iters=20):
             "layers": rows}
 
 
-def grey_field(shape=SHAPE):
+def grey_field(shape=SHAPE, solid=None):
     """Grey-scale workload: the 256^3 pack of the default bench with ns = 1 in
     the spheres and a grey layer ns = 0.25 on pore cells within 1.5 cells of a
     sphere (unresolved roughness), ns = 0 elsewhere."""

@@ -49,8 +49,9 @@ enum { LBM_BC_PERIODIC = 0, LBM_BC_PRESSURE = 1, LBM_BC_VELOCITY = 2 };
 /* Population storage of the fused kernels.  F32 and F64 compute on f itself,
  * as the reference does (F32 reproduces its FP32 rounding bit for bit).  The
  * *_DEV modes compute in FP32 on f - w and rho - 1 (deviation form); F16_DEV and
- * BF16_DEV store each node's populations relative to its own density,
- * g = f - w*rho_node, with rho_node - 1 kept per node in FP32. */
+ * BF16_DEV store populations relative to a fixed reference density,
+ * g = f - w*rho_ref(x): the linear profile between two fixed-pressure x faces,
+ * else 1. */
 enum {
     LBM_STORE_F32 = 0,       /* FP32 f, reference arithmetic */
     LBM_STORE_F16_DEV = 1,   /* FP16 of g * 2^16, deviation-form FP32 collide */
@@ -79,7 +80,7 @@ typedef struct LbmParams {
     int32_t psi_bc[6];       /* TP:35-40: 0 periodic, 1 constant psi */
     double psi_val[6];
     int32_t device;          /* CUDA device ordinal */
-    int32_t block_size;      /* threads per CTA of the step kernel, 0 = default (128 single-phase, 256 two-phase) */
+    int32_t block_size;      /* threads per CTA of the step kernels (at most 128 where those take links), 0 = default (128) */
 } LbmParams;
 
 typedef struct LbmInfo {

@@ -12,15 +12,15 @@
 //
 // Memory layout (HBM): populations in AoSoA-32 chunks (element (n, s) at
 // n + (n >> 5) * 576 + 32 s, lbm_common.cuh) in two buffers (ping-pong),
-// np = n_fluid padded to 64; dense int32 map cell -> node (or -1 for solid),
-// kept L2-resident by a persisting access-policy window (lbm_capi.cu); packed
-// node coordinates.  Per node and step the kernel moves 19 loads + 19 stores
-// of populations (152 B in FP32, 76 B in 16-bit storage), 4 B of coordinates
-// and the neighbour map rows (L1/L2 hits).
+// np = n_fluid padded to 64; neighbour links (lbm_links.cuh).  Per node and step
+// the kernel moves 19 loads + 19 stores of populations (152 B in FP32, 76 B in
+// 16-bit storage) and 9 B of links.  FP64, the staged kernels and LBM_DEBUG
+// builds find their sources through the dense int32 map cell -> node (or -1 for
+// solid) and packed node coordinates instead.
 //
 // Consecutive steps use programmatic dependent launch: a step's CTAs load their
-// coordinates while the previous step drains, then wait for it (+1.5% on the
-// 256^3 pack).  Measured and rejected on the same pack: a persistent
+// links while the previous step drains, then wait for it.  Measured on the map
+// kernel on the 256^3 pack: that +1.5%; rejected, a persistent
 // grid-stride loop with the next node's coordinates prefetched (24.1k against
 // 33.2k MLUPS: the block-ordered launch keeps the active node window compact
 // in L2) and cp.async prefetch of the next node's 19 populations into shared
@@ -35,15 +35,13 @@
 #include "lbm_kernels.cuh"
 #include "lbm_linkgather.cuh"
 
-// Resident 256-thread CTAs per SM requested for the step kernel (caps
-// registers at 65536 / (256 * n)), as measured on the 256^3 pack (MLUPS):
+// Resident 256-thread CTAs per SM requested for the staged kernels (caps
+// registers at 65536 / (256 * n)), as measured on the 256^3 pack with the map
+// kernel (MLUPS):
 //  * FP32 reference arithmetic: 6 (40 registers); 4 with the dense Guo forcing;
-//  * FP32 deviation form: 6 (40 registers, no spill): 35.3k against 34.9k at 5,
-//    forced 37.1k against 36.9k;
-//  * 16-bit codecs: 6 (40 registers, 16-24 bytes spilled): FP16 32.2k / BF16
-//    32.8k against 32.0k / 32.5k at 4 (64 registers) and 29.5k / 30.2k at 5
-//    (48 registers, 68 bytes spilled); forced, 4 is ahead (33.4k / 34.0k
-//    against 33.3k / 33.8k at 6).
+//  * FP32 deviation form: 6 (40 registers, no spill): 35.3k against 34.9k at 5;
+//  * 16-bit codecs: 6 (40 registers): FP16 32.2k / BF16 32.8k against 32.0k /
+//    32.5k at 4 (64 registers) and 29.5k / 30.2k at 5; forced, 4 is ahead.
 #ifndef LBM_SP_MINBLOCKS
 #define LBM_SP_MINBLOCKS 6
 #endif
@@ -126,12 +124,9 @@ __device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int 
                                           lbm_ref_at(sp_ref(C), i), C, fout, vprev, rho_out, v_out);
 }
 
+// The step through the dense map: FP64, and every storage in LBM_DEBUG builds.
 template <int STORE, int FORCE, bool MACROS>
-__global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1
-                                           : Codec<STORE>::RHOREF ? (FORCE ? LBM_SP_MINBLOCKS_16F : LBM_SP_MINBLOCKS_16)
-                                       : Codec<STORE>::DEV    ? LBM_SP_MINBLOCKS_DEV
-                                           : FORCE                ? 4
-                                                                  : LBM_SP_MINBLOCKS)
+__global__ void __launch_bounds__(256)
     sp_step_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C,
                                                       const typename Codec<STORE>::T* __restrict__ fin,
                                                       typename Codec<STORE>::T* __restrict__ fout,
@@ -745,8 +740,6 @@ int run_links(LbmHandle* h, int32_t n, bool macros_last) {
 
 template <int STORE>
 int run_steps(LbmHandle* h, int32_t n, bool macros_last) {
-    using R = typename Codec<STORE>::R;
-    SpConsts<R> C = sp_make_consts<R>(h);
 #ifdef LBM_DEBUG
     int rc0 = lbm_cuda_check(h, cudaMemcpyToSymbolAsync(g_lbm_debug_nlimit, &h->n_fluid, sizeof(int), 0,
                                                         cudaMemcpyHostToDevice, h->stream),
@@ -755,20 +748,27 @@ int run_steps(LbmHandle* h, int32_t n, bool macros_last) {
     if (rc0) return rc0;
 #endif
     if (h->tiled) return run_tiles<STORE>(h, n, macros_last);
-#ifndef LBM_DEBUG
-    // (debug builds keep the kernel whose map lookups they check)
-    if constexpr (STORE != LBM_STORE_F64) return run_links<STORE>(h, n, macros_last);
+#ifdef LBM_DEBUG
+    constexpr bool LINKS = false;   // debug builds keep the kernel whose map lookups they check
+#else
+    constexpr bool LINKS = STORE != LBM_STORE_F64;   // the links gather into FP32
 #endif
-    const int grid = (int)((h->n_fluid + h->block - 1) / h->block);
-    for (int32_t it = 0; it < n; ++it) {
-        const bool mac = macros_last && it == n - 1;
-        C.seed = (uint32_t)(h->steps_done + it);   // global step index: rounding bits of this step
-        int rc;
-        if (h->force) rc = mac ? launch_step<STORE, true, true>(h, C, grid) : launch_step<STORE, true, false>(h, C, grid);
-        else rc = mac ? launch_step<STORE, false, true>(h, C, grid) : launch_step<STORE, false, false>(h, C, grid);
-        if (rc) return rc;
+    if constexpr (LINKS) {
+        return run_links<STORE>(h, n, macros_last);
+    } else {
+        using R = typename Codec<STORE>::R;
+        SpConsts<R> C = sp_make_consts<R>(h);
+        const int grid = (int)((h->n_fluid + h->block - 1) / h->block);
+        for (int32_t it = 0; it < n; ++it) {
+            const bool mac = macros_last && it == n - 1;
+            C.seed = (uint32_t)(h->steps_done + it);   // global step index: rounding bits of this step
+            int rc;
+            if (h->force) rc = mac ? launch_step<STORE, true, true>(h, C, grid) : launch_step<STORE, true, false>(h, C, grid);
+            else rc = mac ? launch_step<STORE, false, true>(h, C, grid) : launch_step<STORE, false, false>(h, C, grid);
+            if (rc) return rc;
+        }
+        return LBM_OK;
     }
-    return LBM_OK;
 }
 
 template <int STORE>
@@ -860,8 +860,8 @@ int sp_launch_init(LbmHandle* h, const void* rho_nodes, const void* v_nodes) {
 }
 
 // Per-tile staging plan of the staged step kernels (after the index is built),
-// chosen by LBM_SP_TILED in the environment: 0 or unset = sp_step_kernel (the
-// default: fastest measured), 1 = persistent staged kernel, 2 = one staged tile
+// chosen by LBM_SP_TILED in the environment: 0 or unset = sp_link_kernel (the
+// default: 36.9k / 38.7k / 40.6k), 1 = persistent staged kernel, 2 = one staged tile
 // per CTA.  256^3 pack, FP32 / f32dev / FP16 MLUPS on one GB300: sp_step_kernel
 // 34.6k / 35.4k / 31.8k; persistent staged 29.2k / 29.9k / 29.4k; one tile per
 // CTA 28.6k / 28.9k / 28.4k, and 32.3k / 32.9k / 29.1k when that kernel stages

@@ -659,40 +659,38 @@ __global__ void __launch_bounds__(TMA_THREADS) conv3d_halo_kernel(const HaloArgs
 
 // ---------------------------------------------------------------------------
 // Warp-specialised weight gradient for layers whose output is one channel part
-// (16, 32 or 64 channels) and whose input is one, or several of 16 (a CTA per
-// part, blockIdx.y): the same GEMM, tap groups, ones
+// (16, 32 or 64 channels) and whose input is one, or several of 16 channels (a CTA
+// per part, blockIdx.y): the same GEMM, tap groups, ones
 // slot and partials as conv3d_wgrad_tma_kernel, but each 8 x 4 x 4 block is
-// loaded once -- one dense TMA box of the 10 x 6 x 6 input halo and one of g
-// (no swizzle) -- and a CTA runs all tap groups of its blocks, one TMEM
+// loaded once -- one dense TMA box of the 10 x 6 x 6 input halo and one of g,
+// swizzled into the B operand's layout -- and a CTA runs all tap groups of its blocks, one TMEM
 // accumulator per group.
 //   last warp, lane 0: TMA producer (two boxes per block, two buffers) and MMA
 //     issuer (8 K = 16 steps per block and group, two operand buffers);
 //   warps 0-7: build the operand buffer of each (block, group) step from the
 //     halo -- tap slot j row r is the halo voxel r shifted by the tap, written
-//     in the swizzled MN-major layout -- and once per block the g operand
-//     (its own two buffers); warps 0-3 run the epilogue.
-// mbarriers between the roles: tfull (TMA -> copy), tempty (copy -> producer,
+//     in the swizzled MN-major layout; warps 0-3 run the epilogue.
+// mbarriers between the roles: tfull (TMA -> copy and MMA), tempty (copy -> producer,
 // WS_COPY arrivals), ofull (copy -> MMA, WS_COPY arrivals), oempty (MMA commit ->
-// copy), done.  Every wait is bounded; a timeout records the error flag and
+// copy and producer), done.  Every wait is bounded; a timeout records the error flag and
 // the roles leave their loops, the producer first waiting (bounded) for the
 // loads it issued.
 // The copies bound it: 64 KB through shared memory a step.  Copy warps and g, us
 // with the partial reduction on 2 x 96^3, 16 -> 16 / 48 -> 16: 4 warps, g with every
-// step 310 / 870; 4 warps, g once a block 299 / 849; 8 warps 230 / 624; 16 warps
-// 397 / 1099 (one CTA per SM).
+// step 310 / 870; 4 warps, g once a block 299 / 849; 8 warps 230 / 624 (16 warps
+// 397 / 1099, one CTA per SM); g as the TMA writes it 227 / 620.
 constexpr int WS_COPY = 256;                     // threads that build operands
 constexpr int WS_THREADS = WS_COPY + 32;
 constexpr int WS_CHUNKS = 2048 / WS_COPY;        // 16-byte pieces of a step's tap slots per thread
 
 struct WsArgs {
     CUtensorMap halo;               // input, tiled 5-D (cin, W, H, D, N), box (cin, 10, 6, 6, 1), no swizzle
-    CUtensorMap gmap;               // g, tiled 5-D (cout, W, H, D, N), box (cout, 8, 4, 4, 1), no swizzle
+    CUtensorMap gmap;               // g, tiled 5-D (cout, W, H, D, N), box (cout, 8, 4, 4, 1), swizzled: the B operand
     int cin, cout, tg, ngroups;     // channels of a part, tap slots per group (128 / cin), groups (ceil(27 / tg))
     int cin_all;                    // channels of the input: cin_all / cin parts, one per blockIdx.y
     uint32_t hbytes;                // bytes of the halo box
-    uint32_t tbytes;                // bytes of one TMA buffer (halo then g), 1024-aligned
+    uint32_t tbytes;                // bytes of one TMA buffer (g then halo), 1024-aligned
     uint32_t obytes;                // bytes of one operand buffer (32 KB of tap slots)
-    uint32_t gbytes;                // bytes of one g operand buffer, 1024-aligned
     uint32_t ncol;                  // TMEM columns (power of two >= ngroups x cout)
     int shift[27];                  // byte offset of tap t's shift inside the halo
     int nbw, nbh, nbd;
@@ -712,7 +710,6 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
     const int tid = threadIdx.x, warp = tid >> 5;
     const uint32_t base = (su32(dsmem) + 1023u) & ~1023u;
     const uint32_t obase = base + 2u * P.tbytes;
-    const uint32_t gbase = obase + 2u * P.obytes;
     const int64_t chunk = blockIdx.x;
     const int64_t b0 = chunk * P.chunk_blocks;
     const int nb = (int)min((int64_t)P.chunk_blocks, P.nblocks - b0);
@@ -762,12 +759,12 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(tx) : "memory");
                 asm volatile(
                     "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                    " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(tb),
+                    " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(tb + 128u * gs),
                     "l"(&P.halo), "r"(part0), "r"(w0 - 1), "r"(h0 - 1), "r"(d0 - 1), "r"(n), "r"(bar)
                     : "memory");
                 asm volatile(
                     "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                    " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(tb + P.hbytes),
+                    " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(tb),
                     "l"(&P.gmap), "r"(0), "r"(w0), "r"(h0), "r"(d0), "r"(n), "r"(bar)
                     : "memory");
             };
@@ -777,10 +774,13 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
             for (int st = 0; st < nsteps && !fail; ++st) {
                 const int b = st / ng, gi = st - b * ng, ob = st & 1;
                 if (!tma_wait(&s_ofull[ob], (uint32_t)((st >> 1) & 1))) { fail = true; break; }
-                if (gi == 0) landed = b + 1;   // the copy warps saw block b's loads complete
+                if (gi == 0) {                 // (the copy warps saw block b's loads complete: returns at once)
+                    if (!tma_wait(&s_tfull[b & 1], (uint32_t)((b >> 1) & 1))) { fail = true; break; }
+                    landed = b + 1;
+                }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t sa = obase + (uint32_t)ob * P.obytes;
-                const uint32_t gb = gbase + (uint32_t)(b & 1) * P.gbytes;
+                const uint32_t gb = base + (uint32_t)(b & 1) * P.tbytes;
                 const uint32_t acc = taddr + (uint32_t)(gi * COUT);
 #pragma unroll 1
                 for (int kk = 0; kk < 8; ++kk) {
@@ -790,8 +790,9 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
                     mma_f16(acc, ad, bdsc, idesc_mn(128, COUT), (b | kk) != 0 ? 1u : 0u);
                 }
                 mma_commit(&s_oempty[ob]);
-                if (gi == ng - 1 && b + 2 < nb) {   // block b's halo is no longer read: load block b + 2 there
-                    if (!tma_wait(&s_tempty[b & 1], (uint32_t)((b >> 1) & 1))) { fail = true; break; }
+                if (gi == ng - 1 && b + 2 < nb) {   // block b's halo and g are no longer read: load block b + 2 there
+                    if (!tma_wait(&s_tempty[b & 1], (uint32_t)((b >> 1) & 1)) ||
+                        !tma_wait(&s_oempty[ob], (uint32_t)((st >> 1) & 1))) { fail = true; break; }
                     issue(b + 2);
                     ++issued;
                 }
@@ -806,7 +807,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
     } else {
         // copy warps: the per-thread chunks of a step are fixed; tap t adds P.shift[t] to the source
         const int csh = pw == 64 ? 3 : (pw == 32 ? 2 : 1);
-        // packed: source offset in the halo (< 46 KB) | destination offset in the tap slots (< 32 KB) << 16
+        // packed: source offset in the TMA buffer (< 64 KB) | destination offset in the tap slots (< 32 KB) << 16
         uint32_t pk[WS_CHUNKS];
 #pragma unroll
         for (int k = 0; k < WS_CHUNKS; ++k) {
@@ -815,11 +816,10 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
             const int r = (e >> csh) & 127;
             const int j = e >> (7 + csh);                     // tap slot (< tg)
             const int x = r & 7, y = (r >> 3) & 3, z = r >> 5;   // voxel of the block; halo origin at -1
-            const uint32_t src = (uint32_t)((z * 6 + y) * 10 + x) * span + (uint32_t)c * 16u;
+            const uint32_t src = 128u * gs + (uint32_t)((z * 6 + y) * 10 + x) * span + (uint32_t)c * 16u;
             const uint32_t dst = (uint32_t)j * 128u * span + swz((uint32_t)r, (uint32_t)c, span);
             pk[k] = src | (dst << 16);
         }
-        const int gch = COUT / 8;                             // g chunks per row
         bool fail = false;
         for (int st = 0; st < nsteps; ++st) {
             const int b = st / ng, gi = st - b * ng, ob = st & 1;
@@ -844,21 +844,9 @@ __global__ void __launch_bounds__(WS_THREADS, 1) conv3d_wgrad_ws_kernel(const __
                     asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(osh + (pk[k] >> 16)), "r"(one) : "memory");
                 }
             }
-            // g operand, once a block (the block two before no longer reads this buffer:
-            // the wait above saw all but its successor's last steps done): row r, chunk c8
-            for (int e = gi == 0 ? tid : 128 * gch; e < 128 * gch; e += WS_COPY) {
-                const int c8 = e % gch, r = e / gch;
-                uint32_t v0, v1, v2, v3;
-                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(v0), "=r"(v1), "=r"(v2), "=r"(v3)
-                             : "r"(tsh + P.hbytes + (uint32_t)r * gs + (uint32_t)c8 * 16u));
-                asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(gbase + (uint32_t)(b & 1) * P.gbytes + swz((uint32_t)r, (uint32_t)c8, gs)),
-                             "r"(v0), "r"(v1), "r"(v2), "r"(v3)
-                             : "memory");
-            }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&s_ofull[ob])) : "memory");
-            if (gi == ng - 1)   // done reading block b's halo and g
+            if (gi == ng - 1)   // done reading block b's halo
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(su32(&s_tempty[b & 1])) : "memory");
         }
         if (fail) {
@@ -1208,18 +1196,21 @@ int nn_wgrad_tma(const void* in, const void* g, float* part, float* dbpart, int 
     return LBM_OK;
 }
 
-// Warp-specialised weight gradient: one-part layers (cin and cout in {16, 32, 64})
-// whose accumulators (groups x cout columns) and buffers fit.  It is taken where
-// two CTAs fit an SM (113 KB) or cout = 64: with one CTA per SM the
-// TMA-box kernel was faster on 16 -> 32 and 32 -> 32 (2 x 48^3), while on 32 -> 64
-// the per-group reload of the 64-channel g made that kernel the slower one.
-// 64 -> 64 runs as four parts of 16 channels (2 x 24^3: 55 us against 77), 48 -> 16
-// as three: 624 us on 2 x 96^3 (partial
-// reduction included) against 1114 with the TMA-box kernel (48 channels in one
-// part need 1598: one CTA per SM).  LBM_NN_WS=0 in the environment turns it off.
+// Warp-specialised weight gradient, taken where two CTAs fit an SM (113 KB) or
+// cout = 64.  Two CTAs fit with parts of 16 input channels and up to 32 outputs,
+// so such layers run as cin / 16 parts; us with the partial reduction, parts against
+// the TMA-box kernel: 2 x 96^3 16 -> 16 227 / 449, 32 -> 16 431 / 687, 48 -> 16 620 /
+// 1114; 2 x 48^3 64 -> 16 167 / 205, 96 -> 16 247 / 279, 16 -> 32 58 / 87, 32 -> 32
+// 111 / 146, 64 -> 32 207 / 209, 80 -> 32 250 / 283; 2 x 24^3 128 -> 32 56 / 78.
+// 48 -> 32 and 96 -> 32 stay with the box kernel (168 / 160, 301 / 279: its parts
+// of 32 + 16 and 64 + 32 channels leave no slot empty).  One CTA per SM: 64 -> 64 as
+// four parts (2 x 24^3 54 / 77), 32 -> 64 whole (33; two parts 39).
+// LBM_NN_WS=0 in the environment turns it off.
 static bool ws_plan(int cin_all, int cout, WsArgs* P, size_t* smem) {
     // channels of a part
-    const int cin = (cin_all == 48 && cout == 16) || (cin_all == 64 && cout == 64) ? 16 : cin_all;
+    const bool parts = cin_all % 16 == 0 && cin_all <= 128 && cin_all != 112 &&   // what the box kernel takes
+                       (cout == 16 || (cout == 32 && cin_all % 48 != 0) || (cout == 64 && cin_all == 64));
+    const int cin = parts ? 16 : cin_all;
     P->cin_all = cin_all;
     if (!(cin == 16 || cin == 32 || cin == 64) || !(cout == 16 || cout == 32 || cout == 64)) return false;
     P->cin = cin;
@@ -1232,9 +1223,8 @@ static bool ws_plan(int cin_all, int cout, WsArgs* P, size_t* smem) {
     P->hbytes = 360u * (uint32_t)cin * 2u;
     P->tbytes = (P->hbytes + 128u * 2u * (uint32_t)cout + 1023u) & ~1023u;
     P->obytes = 32768u;
-    P->gbytes = (128u * 2u * (uint32_t)cout + 1023u) & ~1023u;
     for (int t = 0; t < 27; ++t) P->shift[t] = ((t / 9) * 60 + ((t / 3) % 3) * 10 + t % 3) * cin * 2;
-    *smem = 2 * ((size_t)P->tbytes + P->obytes + P->gbytes) + 1024;
+    *smem = 2 * ((size_t)P->tbytes + P->obytes) + 1024;
     return *smem <= 227 * 1024;
 }
 
@@ -1291,7 +1281,7 @@ int nn_wgrad_ws(const void* in, const void* g, float* part, float* dbpart, int n
                                    (cuuint64_t)d * h * wd * cout * 2};
         const cuuint32_t box[5] = {(cuuint32_t)cout, WGB_W, WGB_H, WGB_D, 1};
         const CUresult r = g_enc_tiled(&P.gmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(g), dim, str, box,
-                                       es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                       es, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_of(2 * cout),
                                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS)
             return lbm_set_err(nullptr, LBM_ECUDA, "lbm_nn_conv3d_wgrad (ws): g tensor map, error " + std::to_string((int)r));

@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(256)
 // 35.5k / 36.9k, FP32 deviation form 35.1k / 36.1k / 38.7k, FP16 32.2k / 39.9k /
 // 40.6k; 64^3 cavity FP32 30.1k / 34.3k / 33.7k (launch-bound); channel 101 x 67 x 53,
 // FP32 forced along x 19.3k / 21.3k / 28.7k (with the x-only Guo term).
-// FP32 then moves 166 B a node at 0.93 of the copy bandwidth (DRAM-bound); the
+// FP32 then moves 167 B a node at 0.92 of the copy bandwidth (DRAM-bound); the
 // 16-bit storages are bound by issue slots (87% of them used).  Two nodes per
 // thread in packed FP32 halve the instructions and were slower (28.0k FP32, 96
 // registers: half the warps, each living longer), pushing instead of pulling

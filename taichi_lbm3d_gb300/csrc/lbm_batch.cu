@@ -425,8 +425,13 @@ int lbm_batch_configure(LbmBatch* b, const int32_t* tile_len, int32_t block) {
         b->tile_len[q] = tile_len[q];
     }
     b->block = block;
-    destroy_graph(b);
-    return LBM_OK;
+    if (b->tiles.empty()) {
+        destroy_graph(b);
+        return LBM_OK;
+    }
+    // the kernel has a thread for every node of a tile: tiles in use are cut again
+    cudaSetDevice(b->h.device);
+    return rebuild_tiles(b);
 }
 
 int lbm_batch_init(LbmBatch* b) {

@@ -60,6 +60,7 @@ struct LbmBatch {
     int32_t graph_steps = 0;
     std::vector<int64_t> steps;         // per subvolume
     uint32_t seed_step = 0;             // steps taken since init (16-bit rounding seed)
+    bool initialized = false;
 };
 
 namespace {
@@ -425,10 +426,7 @@ int lbm_batch_configure(LbmBatch* b, const int32_t* tile_len, int32_t block) {
         b->tile_len[q] = tile_len[q];
     }
     b->block = block;
-    if (b->tiles.empty()) {
-        destroy_graph(b);
-        return LBM_OK;
-    }
+    if (!b->initialized) return LBM_OK;
     // the kernel has a thread for every node of a tile: tiles in use are cut again
     cudaSetDevice(b->h.device);
     return rebuild_tiles(b);
@@ -452,6 +450,7 @@ int lbm_batch_init(LbmBatch* b) {
     if (!rc) rc = rebuild_tiles(b);
     b->seed_step = 0;
     destroy_graph(b);
+    b->initialized = rc == LBM_OK;
     return rc;
 }
 
@@ -491,6 +490,7 @@ static int batch_run(LbmBatch* b, int32_t nsteps, int32_t chunk, int32_t use_gra
 
 int lbm_batch_step(LbmBatch* b, int32_t nsteps, int32_t chunk, int32_t use_graph) {
     if (!b) return lbm_set_err(nullptr, LBM_EINVAL, "lbm_batch_step: NULL");
+    if (!b->initialized) return batch_err(b, LBM_ESTATE, "lbm_batch_step: call lbm_batch_init first");
     if (chunk < 2 || chunk > 4096 || chunk % 2 || nsteps % chunk)
         return batch_err(b, LBM_EINVAL, "lbm_batch_step: chunk must be even, <= 4096, and divide nsteps");
     cudaSetDevice(b->h.device);
@@ -526,6 +526,7 @@ int lbm_batch_run_to_convergence(LbmBatch* b, double tol, int32_t check_every, i
     if (!b || !darcy || !steps || !converged) return lbm_set_err(nullptr, LBM_EINVAL, "lbm_batch_run_to_convergence: NULL");
     if (check_every < 2 || check_every > 4096 || check_every % 2)
         return batch_err(b, LBM_EINVAL, "lbm_batch_run_to_convergence: check_every must be even and <= 4096");
+    if (!b->initialized) return batch_err(b, LBM_ESTATE, "lbm_batch_run_to_convergence: call lbm_batch_init first");
     LbmHandle* h = &b->h;
     cudaSetDevice(h->device);
     const size_t ns = b->subs.size();

@@ -37,3 +37,29 @@ def test_configure_after_init_and_between_steps(tile, block, use_graph):
     b.step(4, chunk=2, use_graph=use_graph)
     assert all(np.array_equal(x, y) for x, y in zip(fields(b), ref))
     b.close()
+
+
+@pytest.mark.parametrize("call", [lambda b: b.step(4, chunk=2), lambda b: b.step(4, chunk=2, use_graph=False),
+                                  lambda b: b.run_to_convergence(check_every=2, max_steps=8)])
+def test_steps_before_init_are_refused(call):
+    """Without a state there is nothing to step; a zero Darcy velocity would read as converged."""
+    from taichi_lbm3d_gb300 import _native
+    b = batch()
+    with pytest.raises(_native.LbmError):
+        call(b)
+    b.configure([64, 64], 64)
+    b.init()
+    call(b)
+    b.close()
+
+
+@pytest.mark.parametrize("storage", ["f32", "f16"])
+def test_batch_without_any_fluid(storage):
+    from taichi_lbm3d_gb300.batch import Batch
+    b = Batch([np.ones((9, 7, 5), np.int8)], storage=storage)
+    b.init()
+    b.step(4, chunk=2)
+    darcy, steps, conv = b.run_to_convergence(check_every=2, max_steps=8)
+    rho, v = b.macros(0)
+    b.close()
+    assert darcy[0] == 0.0 and conv[0] and np.all(rho == 1.0) and np.all(v == 0.0)

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Co
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int4 t4 = __ldg(reinterpret_cast<const int4*>(tiles + blockIdx.x));
     const int64_t first = (int64_t)t4.x * 32;
-    const LbmLinks L{links.node + first, links.head + t4.x, links.rec0 + t4.x, links.rec};
+    const LbmLinks L{links.node + first, links.head + t4.x, links.recs + t4.x, links.rec};
     const int n = t4.y + threadIdx.x;
     const bool live = n < t4.z;
     NodeLinks K;

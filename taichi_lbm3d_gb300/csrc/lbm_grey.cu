@@ -106,8 +106,8 @@ __global__ void __launch_bounds__(GREY_THREADS, STORE == LBM_STORE_F64 ? 2 : 8) 
     if (n >= C.n_fluid) return;
     NodeLinks K;
     K.load(L, n);
-    const int32_t* rec = L.rec;
-    const bool exc = K.record(L, n, rec);
+    const bool exc = K.any_record();
+    const int32_t* rec = K.bits & LBM_LINK_EXC ? K.record(L, n) : L.rec;
     const bool on = K.bits & LBM_LINK_FACE;
     int i = 0, j = 0, k = 0;
     if (Cd::RHOREF || on) {

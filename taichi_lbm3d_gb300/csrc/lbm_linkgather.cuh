@@ -61,14 +61,15 @@ struct NodeLinks {
             return rank<rw>();
         }
     }
-    // Whether any node of the warp (one group) has a record; this node's.
-    __device__ __forceinline__ bool record(const LbmLinks& L, int n, const int32_t*& rec) const {
-        const uint32_t e = __ballot_sync(__activemask(), bits & LBM_LINK_EXC);
-        if (e)
-            rec = L.rec + (int64_t)LBM_LINK_REC *
-                              (__ldg(L.rec0 + n / LBM_LINK_GROUP) + __popc(e & ((1u << (threadIdx.x & 31)) - 1u)));
-        return e != 0;
+    // The node's record, for nodes that have one (LBM_LINK_EXC): found without a
+    // vote, since which lanes are together at a vote is not fixed.
+    __device__ __forceinline__ const int32_t* record(const LbmLinks& L, int n) const {
+        const int2 r = __ldg(reinterpret_cast<const int2*>(L.recs + n / LBM_LINK_GROUP));
+        return L.rec + (int64_t)LBM_LINK_REC * (r.x + __popc((uint32_t)r.y & ((1u << lane) - 1u)));
     }
+    // Whether to take the code that looks for records: it serves every node, the
+    // code without only those that have none.
+    __device__ __forceinline__ bool any_record() const { return __any_sync(__activemask(), bits & LBM_LINK_EXC); }
 };
 
 // Reference density of the 16-bit codecs at a node and its sources at x - 1 and
@@ -116,12 +117,11 @@ struct LinkGather {
         F[S] = get<S>(fin[a + 32 * S]);
         if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), bounce ? rx.at : rx.template of<S>(), F[S]);
     }
-    // Explicit sources of the links that the node word cannot express; a warp
-    // holds one group.
+    // Explicit sources of the links that the node word cannot express.
     static __device__ __forceinline__ void recorded(R* F, const T* fin, const LbmLinks& L, const NodeLinks& K, int n,
                                                     const LinkRef<R>& rx) {
-        const int32_t* rec = L.rec;
-        if (!K.record(L, n, rec) || !(K.bits & LBM_LINK_EXC)) return;
+        if (!(K.bits & LBM_LINK_EXC)) return;
+        const int32_t* rec = K.record(L, n);
 #define LBM_X(S)                                                                              \
     {                                                                                         \
         const int src = __ldg(rec + S);                                                       \

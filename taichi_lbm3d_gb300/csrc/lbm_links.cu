@@ -20,7 +20,7 @@ struct LinkBuild {
     int32_t every;        // records on replaced nodes too (two phases: the colours are pulled there)
     uint2* node;
     LbmLinkHead* head;
-    int32_t* rec0;
+    LbmLinkRecs* recs;
     int32_t* rec;
     int32_t cap;          // records allocated
     int32_t* total;       // records needed
@@ -123,10 +123,10 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
         for (int r = 1; r < 8; ++r)
             if (lane == r) v = start[r];
         if (lane < 8) B.head[group].start[lane] = v;
-        if (lane == 0) B.rec0[group] = exc ? atomicAdd(B.total, __popc(exc)) : 0;
+        if (lane == 0) B.recs[group] = {exc ? atomicAdd(B.total, __popc(exc)) : 0, exc};
         B.node[n] = make_uint2(w0, w1 | bits);
     } else if (bits & LBM_LINK_EXC) {
-        const int slot = B.rec0[group] + __popc(exc & ((1u << lane) - 1u));
+        const int slot = B.recs[group].first + __popc(exc & ((1u << lane) - 1u));
         if (slot >= B.cap) return;               // the host allocates more and builds again
         int32_t* out = B.rec + (int64_t)LBM_LINK_REC * slot;
         out[0] = out[19] = -1;
@@ -162,8 +162,8 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
     }
     for (;;) {
         const size_t node = sizeof(uint2) * h->np, head = sizeof(LbmLinkHead) * ngroup;
-        const size_t rec0 = (sizeof(int32_t) * (ngroup + 1) + 15) / 16 * 16;   // + the count
-        const size_t bytes = node + head + rec0 + sizeof(int32_t) * LBM_LINK_REC * cap;
+        const size_t recs = (sizeof(LbmLinkRecs) * (ngroup + 1) + 15) / 16 * 16;   // + the count
+        const size_t bytes = node + head + recs + sizeof(int32_t) * LBM_LINK_REC * cap;
         int rc = lbm_cuda_check(h, cudaMalloc(&h->d_links, bytes), "neighbour links");
         if (rc) {
             h->d_links = nullptr;
@@ -171,9 +171,9 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
         }
         h->device_bytes += (int64_t)bytes;
         char* at = (char*)h->d_links;
-        const LbmLinks L{(uint2*)at, (LbmLinkHead*)(at + node), (int32_t*)(at + node + head), (int32_t*)(at + node + head + rec0)};
+        const LbmLinks L{(uint2*)at, (LbmLinkHead*)(at + node), (LbmLinkRecs*)(at + node + head), (int32_t*)(at + node + head + recs)};
         h->links = L;
-        int32_t* d_total = (int32_t*)(at + node + head) + ngroup;
+        int32_t* d_total = (int32_t*)(L.recs + ngroup);
         rc = lbm_cuda_check(h, cudaMemsetAsync(d_total, 0, sizeof(int32_t), h->stream), "link records");
         if (rc) return rc;
         for (int pass = 0; pass < 2; ++pass)
@@ -189,7 +189,7 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
                 B.every = p.two_phase;
                 B.node = (uint2*)L.node + l.node_begin;
                 B.head = (LbmLinkHead*)L.head + l.node_begin / LBM_LINK_GROUP;
-                B.rec0 = (int32_t*)L.rec0 + l.node_begin / LBM_LINK_GROUP;
+                B.recs = (LbmLinkRecs*)L.recs + l.node_begin / LBM_LINK_GROUP;
                 B.rec = (int32_t*)L.rec;
                 B.cap = (int32_t)cap;
                 B.total = d_total;

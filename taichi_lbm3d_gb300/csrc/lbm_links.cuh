@@ -9,7 +9,7 @@
 // other rows keeps close to a straight line: LbmLinkHead holds its start, a node
 // word the 5-bit distance of its rank from start + lane and one bit per direction
 // "take the own opposite slot" (solid source: halfway bounce-back).  That is 9
-// bytes a node (8 + 32 per 32 nodes), read in order, in the place of 18 lookups
+// bytes a node (8 + 32 per 32 nodes; LbmLinkRecs is read by nodes with a record), read in order, in the place of 18 lookups
 // in the dense map (4 bytes a cell in three z planes, behind a load of the
 // coordinates).  On sphere packs of porosity 0.25 to 0.5 the 5 bits fall short
 // in 0.1% to 0.3% of the groups of 32 nodes (8 bits cost 3.5 bytes a node more).
@@ -18,7 +18,8 @@
 // more than 31 from the row's line, has its bit set too, the node's LBM_LINK_EXC
 // bit is set, and an explicit record of 20 int32 holds the source of each such
 // direction (-1 in the others).  Records of 32 nodes are consecutive in node
-// order from rec0.  Single-phase nodes whose populations a face condition
+// order; LbmLinkRecs has the first one and the lanes that have one, so that a node
+// finds its own without asking the other lanes.  Single-phase nodes whose populations a face condition
 // replaces whole need none for what they pull.
 #pragma once
 #include <cuda_runtime.h>
@@ -37,10 +38,15 @@ struct __align__(16) LbmLinkHead {
     int32_t start[8];  // rows ordered as lbm_link_ey / lbm_link_ez
 };
 
+struct __align__(8) LbmLinkRecs {
+    int32_t first;     // first record of the group
+    uint32_t lanes;    // its nodes that have one
+};
+
 struct LbmLinks {
     const uint2* node;            // [np]
     const LbmLinkHead* head;      // [np / 32]
-    const int32_t* rec0;          // [np / 32] first record of the group
+    const LbmLinkRecs* recs;      // [np / 32]
     const int32_t* rec;           // LBM_LINK_REC per record
 };
 

@@ -357,8 +357,8 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : LBM_TP_MINBLOCKS_A) 
     if (n >= T.sp.n_fluid) return;
     NodeLinks K;
     K.load(L, n);
-    const int32_t* rec = L.rec;
-    const bool exc = K.record(L, n, rec);
+    const bool exc = K.any_record();
+    const int32_t* rec = K.bits & LBM_LINK_EXC ? K.record(L, n) : L.rec;
     // records and amounts of the previous flow launch; psi is rewritten below
     const ColourRec<R>* crec = wait_previous(crec_prev);
     const R* vz = launder(vz_prev);

@@ -213,10 +213,26 @@ bool step_graph_pays(LbmHandle* h, int32_t n) {
 #endif
 }
 
+// While it lives, this thread's calls are not held against a capture that the
+// caller, or another thread, has under way in the global mode: instantiating a
+// graph would otherwise end that capture with an error.
+struct CaptureRelaxed {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    CaptureRelaxed() {
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) cudaGetLastError();
+    }
+    ~CaptureRelaxed() {
+        if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) cudaGetLastError();
+    }
+    CaptureRelaxed(const CaptureRelaxed&) = delete;
+    CaptureRelaxed& operator=(const CaptureRelaxed&) = delete;
+};
+
 // 0: launched; 1: could not be captured (the steps are launched one by one); < 0: error.
 int step_graph_launch(LbmHandle* h) {
     cudaGraphExec_t& exec = h->step_graph[h->cur];
     if (!exec) {
+        const CaptureRelaxed relaxed;
         if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
             cudaGetLastError();
             return 1;

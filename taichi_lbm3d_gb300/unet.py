@@ -333,7 +333,10 @@ class UNet3D:
         items += [(self.hw, hw_hb_g[:OUT * 16].view(OUT, 16), None), (self.hb, hw_hb_g[OUT * 16:], None)]
         shape = {name: (cin, cout) for name, cin, cout, _ in LAYERS}
         rows = (_AdamTensor * len(items))()
+        held = []          # contiguous copies of strided gradients, until the launch is in the stream
         for r, (p, g, name) in zip(rows, items):
+            g = g.contiguous()
+            held.append(g)
             key = p.data_ptr()
             if key not in self.adam:
                 self.adam[key] = (self.torch.zeros_like(p), self.torch.zeros_like(p))

@@ -19,8 +19,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <exception>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -223,39 +223,58 @@ static bool resident(char* p, size_t n) {
     return true;
 }
 
+// Whether p is ordinary host memory, whose pages are this thread's to touch
+// (the outputs may lie in pinned, managed or device memory too).
+static bool pageable(const void* p) {
+    cudaPointerAttributes a = {};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
 // A fresh host array costs a page fault per page on its first write, and the
 // copy's single thread takes them one after another (a 256^3 rho and v: most of
 // 15 ms).  Up to 8 threads touch the pages while the GPU lays the values out:
 // 300 steps and readback of the 256^3 FP32 pack 62.0 -> 53.5 ms.  Arrays that the
 // allocator hands out again (below its mmap threshold) have their pages already and
 // are left alone (rho and v of 150 x 131 x 97: 840 us with the touch, 420 without).
+// Without memory or threads for it the pages are left to the copy.
 void host_touch(void* const* p, const size_t* bytes, int count) {
     constexpr size_t PAGE = 4096, PIECE = (size_t)4 << 20;
+    constexpr unsigned MOST = 8;
     struct Span {
         char* at;
         size_t n;
     };
-    std::vector<Span> work;
-    for (int q = 0; q < count; ++q)
-        for (size_t o = 0; p[q] && o < bytes[q]; o += PIECE) {
-            const size_t n = std::min(PIECE, bytes[q] - o);
-            if (!resident((char*)p[q] + o, n)) work.push_back({(char*)p[q] + o, n});
-        }
-    if (work.size() < 2) return;   // not worth a thread
-    std::atomic<size_t> next{0};
-    auto run = [&] {
-        for (size_t k; (k = next.fetch_add(1)) < work.size();)
-            for (size_t o = 0; o < work[k].n; o += PAGE) *(volatile char*)(work[k].at + o) = 0;
-    };
-    const unsigned n = std::min<unsigned>({8u, std::max(1u, std::thread::hardware_concurrency()), (unsigned)work.size()});
-    std::vector<std::thread> pool;
+    std::thread pool[MOST - 1];
     try {
-        for (unsigned t = 1; t < n; ++t) pool.emplace_back(run);
-    } catch (const std::system_error&) {
-        // fewer threads, or none: this one goes through the rest
+        std::vector<Span> work;
+        for (int q = 0; q < count; ++q) {
+            if (!p[q] || bytes[q] < PIECE || !pageable(p[q])) continue;
+            for (size_t o = 0; o < bytes[q]; o += PIECE) {
+                const size_t n = std::min(PIECE, bytes[q] - o);
+                if (!resident((char*)p[q] + o, n)) work.push_back({(char*)p[q] + o, n});
+            }
+        }
+        if (work.size() < 2) return;   // not worth a thread
+        std::atomic<size_t> next{0};
+        auto run = [&] {
+            for (size_t k; (k = next.fetch_add(1)) < work.size();)
+                for (size_t o = 0; o < work[k].n; o += PAGE) *(volatile char*)(work[k].at + o) = 0;
+        };
+        const unsigned n = std::min<unsigned>({MOST, std::max(1u, std::thread::hardware_concurrency()), (unsigned)work.size()});
+        try {
+            for (unsigned t = 1; t < n; ++t) pool[t - 1] = std::thread(run);
+        } catch (const std::exception&) {
+            // fewer threads, or none: this one goes through the rest
+        }
+        run();
+        for (auto& t : pool)
+            if (t.joinable()) t.join();
+    } catch (const std::exception&) {
     }
-    run();
-    for (auto& t : pool) t.join();
 }
 
 // Dense host arrays from node-ordered device arrays.  The population buffer that

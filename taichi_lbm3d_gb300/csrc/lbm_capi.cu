@@ -422,15 +422,14 @@ int lbm_set_grey(LbmHandle* h, const double* ns) {
         rc = dev_alloc(h, &h->d_gstale, rb * 19 * 2 * (size_t)h->p.ny * h->p.nz, "grey face slots");
     if (!rc) rc = lbm_cuda_check(h, cudaMemcpyAsync(h->d_ns, host.data(), host.size(), cudaMemcpyHostToDevice, h->stream), "copy ns");
     if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "lbm_set_grey");
+    if (!rc && !h->d_links) {   // FP64
+        const LbmLinkLattice lat{h->p.nx, h->p.ny, h->p.nz, h->n_fluid, 0, 0};
+        rc = links_build(h, &lat, 1);
+    }
     if (rc) {
         dev_free(h->d_ns);
         dev_free(h->d_gstale);
         return rc;
-    }
-    if (!h->d_links) {   // FP64
-        const LbmLinkLattice lat{h->p.nx, h->p.ny, h->p.nz, h->n_fluid, 0, 0};
-        rc = links_build(h, &lat, 1);
-        if (rc) return rc;
     }
     h->grey = true;
     return LBM_OK;

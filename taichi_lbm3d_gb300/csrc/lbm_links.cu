@@ -160,10 +160,18 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
             if (p.two_phase || p.bc[f] == LBM_BC_PERIODIC || (p.bc[f] == LBM_BC_VELOCITY && p.bc_form != 0)) seam += area[f / 2];
         cap += std::min<int64_t>(seam, l.n_fluid) + l.n_fluid / 512;
     }
+    size_t bytes = 0;
+    auto drop = [&](int code) {
+        cudaFree(h->d_links);
+        h->d_links = nullptr;
+        h->links = LbmLinks{};
+        h->device_bytes -= (int64_t)bytes;
+        return code;
+    };
     for (;;) {
         const size_t node = sizeof(uint2) * h->np, head = sizeof(LbmLinkHead) * ngroup;
         const size_t recs = (sizeof(LbmLinkRecs) * (ngroup + 1) + 15) / 16 * 16;   // + the count
-        const size_t bytes = node + head + recs + sizeof(int32_t) * LBM_LINK_REC * cap;
+        bytes = node + head + recs + sizeof(int32_t) * LBM_LINK_REC * cap;
         int rc = lbm_cuda_check(h, cudaMalloc(&h->d_links, bytes), "neighbour links");
         if (rc) {
             h->d_links = nullptr;
@@ -175,7 +183,7 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
         h->links = L;
         int32_t* d_total = (int32_t*)(L.recs + ngroup);
         rc = lbm_cuda_check(h, cudaMemsetAsync(d_total, 0, sizeof(int32_t), h->stream), "link records");
-        if (rc) return rc;
+        if (rc) return drop(rc);
         for (int pass = 0; pass < 2; ++pass)
             for (int q = 0; q < count; ++q) {
                 const LbmLinkLattice& l = lat[q];
@@ -203,10 +211,9 @@ int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
         int32_t total = 0;
         if (!rc) rc = lbm_cuda_check(h, cudaMemcpyAsync(&total, d_total, sizeof(int32_t), cudaMemcpyDeviceToHost, h->stream), "link records");
         if (!rc) rc = lbm_cuda_check(h, cudaStreamSynchronize(h->stream), "neighbour links");
-        if (rc || total <= cap) return rc;
-        cudaFree(h->d_links);
-        h->d_links = nullptr;
-        h->device_bytes -= (int64_t)bytes;
+        if (rc) return drop(rc);
+        if (total <= cap) return LBM_OK;
+        drop(LBM_OK);
         cap = total;
     }
 }

@@ -26,8 +26,8 @@ extern "C" int run(int fail, int* kept, long long* bytes, int* live) {
     g_fail = fail;
     LbmHandle h;
     h.p = LbmParams();
-    h.np = 64;
-    const LbmLinkLattice lat{8, 4, 2, 0, 0, 0};   // no fluid: no launch
+    h.np = 0;                                     // no fluid, no groups: nothing is launched
+    const LbmLinkLattice lat{8, 4, 2, 0, 0, 0};
     const int rc = links_build(&h, &lat, 1);
     *kept = h.d_links != nullptr;
     *bytes = h.device_bytes;

@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(GREY_THREADS, STORE == LBM_STORE_F64 ? 2 : 8) 
     NodeLinks K;
     K.load(L, n);
     const bool exc = K.any_record();
-    const int32_t* rec = K.bits & LBM_LINK_EXC ? K.record(L, n) : L.rec;
+    const int32_t* rec = K.record(L);
     const bool on = K.bits & LBM_LINK_FACE;
     int i = 0, j = 0, k = 0;
     if (Cd::RHOREF || on) {

@@ -28,13 +28,15 @@ struct LinkBuild {
 
 struct Row {
     int src[3];           // sources at x - 1, x, x + 1 (wrapped), -1 solid
-    bool cross[3];        // the link crosses a periodic face
+    bool cross[3];        // the link crosses a periodic x face
     int rank;             // rank of the cell across, -1 when no link of the row needs it
 };
 
 // Links of the row (e_y, e_z) of a node; WIDE: the row's three cells, else the one across.
+// A row across a periodic y or z face is a row like any other; of a whole node, whose
+// pulls are replaced, it counts as crossed, so that it does not bend the group's line.
 template <bool WIDE>
-__device__ __forceinline__ Row link_row(const LinkBuild& B, int ey, int ez, int i, int j, int k) {
+__device__ __forceinline__ Row link_row(const LinkBuild& B, int ey, int ez, int i, int j, int k, bool whole) {
     const int y = j - ey, z = k - ez;
     const int yw = y < 0 ? B.ny - 1 : (y >= B.ny ? 0 : y), zw = z < 0 ? B.nz - 1 : (z >= B.nz ? 0 : z);
     const int64_t row = (int64_t)B.nx * (yw + (int64_t)B.ny * zw);
@@ -47,7 +49,7 @@ __device__ __forceinline__ Row link_row(const LinkBuild& B, int ey, int ez, int 
         if (!WIDE && d != 1) continue;
         const int x = i + d - 1;
         const int xw = x < 0 ? B.nx - 1 : (x >= B.nx ? 0 : x);
-        o.cross[d] = x != xw || y != yw || z != zw;
+        o.cross[d] = x != xw || (whole && (y != yw || z != zw));
         o.src[d] = __ldg(B.map + row + xw);
     }
     if (o.src[1] >= 0 && !o.cross[1]) o.rank = o.src[1];
@@ -78,7 +80,7 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
             whole |= !B.every && (B.bc[f] == LBM_BC_PRESSURE || B.bc_form == 0);
         }
         if (at[0] || at[1] || at[2] || at[3] || at[4] || at[5]) bits |= LBM_LINK_EDGE;
-        own = link_row<true>(B, 0, 0, i, j, k);
+        own = link_row<true>(B, 0, 0, i, j, k, whole);
 #pragma unroll
         for (int d = 0; d < 3; d += 2) {
             if (own.src[d] < 0 || own.cross[d]) bits |= d ? 4u : 2u;
@@ -91,8 +93,8 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
     for (int r = 0; r < 8; ++r) {
         int rank = -1;
         if (live) {
-            const Row o = r < 4 ? link_row<true>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k)
-                                : link_row<false>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k);
+            const Row o = r < 4 ? link_row<true>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k, whole)
+                                : link_row<false>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k, whole);
             rank = o.rank;
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
@@ -134,7 +136,7 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
         out[2] = own.cross[2] ? own.src[2] : -1;
 #pragma unroll 1
         for (int r = 0; r < 8; ++r) {
-            const Row o = link_row<true>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k);
+            const Row o = link_row<true>(B, lbm_link_ey(r), lbm_link_ez(r), i, j, k, whole);
 #pragma unroll
             for (int d = 0; d < 3; ++d)
                 if (r < 4 || d == 1) out[lbm_link_dir(r, 1 - d)] = o.cross[d] || (far >> r & 1u) ? o.src[d] : -1;
@@ -146,15 +148,16 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
 
 // Links of `count` lattices whose maps and coordinates lie in h->d_map and
 // h->d_coord (node numbers local to each lattice); one allocation
-// (h->d_links).  Records: room for every node of the periodic faces; geometries
-// that need more (rows far from a line) get a second one.
+// (h->d_links).  Records: room for every node of the periodic x faces and for the
+// groups where a row starts anew across a y or z face; geometries that need more
+// (rows far from a line) get a second one.
 int links_build(LbmHandle* h, const LbmLinkLattice* lat, int count) {
     const LbmParams& p = h->p;
     const int64_t ngroup = h->np / LBM_LINK_GROUP;
     int64_t cap = 32;
     for (int q = 0; q < count; ++q) {
         const LbmLinkLattice& l = lat[q];
-        const int64_t area[3] = {(int64_t)l.ny * l.nz, (int64_t)l.nx * l.nz, (int64_t)l.nx * l.ny};
+        const int64_t area[3] = {(int64_t)l.ny * l.nz, LBM_LINK_GROUP * (int64_t)l.nz, LBM_LINK_GROUP};
         int64_t seam = 0;
         for (int f = 0; f < 6; ++f)
             if (p.two_phase || p.bc[f] == LBM_BC_PERIODIC || (p.bc[f] == LBM_BC_VELOCITY && p.bc_form != 0)) seam += area[f / 2];

@@ -14,8 +14,9 @@
 // coordinates).  On sphere packs of porosity 0.25 to 0.5 the 5 bits fall short
 // in 0.1% to 0.3% of the groups of 32 nodes (8 bits cost 3.5 bytes a node more).
 //
-// A link that this cannot express, i.e. one that crosses a periodic face or is
-// more than 31 from the row's line, has its bit set too, the node's LBM_LINK_EXC
+// A link that this cannot express, i.e. one that crosses a periodic x face or is
+// more than 31 from the row's line (as where 32 nodes lie on both sides of a periodic
+// y or z face's first row), has its bit set too, the node's LBM_LINK_EXC
 // bit is set, and an explicit record of 20 int32 holds the source of each such
 // direction (-1 in the others).  Records of 32 nodes are consecutive in node
 // order; LbmLinkRecs has the first one and the lanes that have one, so that a node

@@ -358,7 +358,7 @@ __global__ void __launch_bounds__(128, sizeof(R) == 8 ? 4 : LBM_TP_MINBLOCKS_A) 
     NodeLinks K;
     K.load(L, n);
     const bool exc = K.any_record();
-    const int32_t* rec = K.bits & LBM_LINK_EXC ? K.record(L, n) : L.rec;
+    const int32_t* rec = K.record(L);
     // records and amounts of the previous flow launch; psi is rewritten below
     const ColourRec<R>* crec = wait_previous(crec_prev);
     const R* vz = launder(vz_prev);

@@ -21,14 +21,14 @@ using namespace lbmk;
 __global__ void index_kernel(LbmLinks L, int split, int* out) {
     const int n = blockIdx.x * 32 + threadIdx.x;
     NodeLinks K;
-    K.load(L, n);
-    if (!(K.bits & LBM_LINK_EXC)) return;
     if (n % split == 0) {
-        out[n] = (int)((K.record(L, n) - L.rec) / LBM_LINK_REC);
+        K.load(L, n);
+        if (K.bits & LBM_LINK_EXC) out[n] = (int)((K.record(L) - L.rec) / LBM_LINK_REC);
         __threadfence();
     } else {
         __nanosleep(200);
-        out[n] = (int)((K.record(L, n) - L.rec) / LBM_LINK_REC);
+        K.load(L, n);
+        if (K.bits & LBM_LINK_EXC) out[n] = (int)((K.record(L) - L.rec) / LBM_LINK_REC);
     }
 }
 extern "C" int record_index(const void* node, const void* head, const void* recs, int groups, int split, int* out) {
@@ -85,3 +85,39 @@ def test_partial_last_group(n, two_phase):
     fl = solid == 0
     for f, g in got.items():
         assert np.array_equal(g[fl], o.field(f).astype(np.float32)[fl], equal_nan=True), f
+
+
+@pytest.mark.parametrize("shape", [(70, 9, 1), (9, 70, 1), (33, 1, 5), (40, 37, 2), (5, 7, 3), (16, 8, 8), (24, 6, 9),
+                                   (1, 9, 9), (2, 5, 5), (1, 1, 40)])
+@pytest.mark.parametrize("bc,bc_form", [((0,) * 6, 0), ((0, 0, 1, 0, 0, 0), 0), ((0, 0, 0, 2, 0, 0), 1),
+                                        ((1, 1, 0, 0, 0, 0), 0), ((0, 0, 0, 0, 2, 1), 0)])
+@pytest.mark.parametrize("dense", [0.0, 0.3])
+def test_rows_across_seams(shape, bc, bc_form, dense):
+    """Rows across periodic y and z faces, alone and beside fixed faces, bit for bit."""
+    if any(bc[f] and shape[f // 2] < 2 for f in range(6)):
+        pytest.skip("a fixed face needs two cells")
+    solid = (np.random.default_rng(7).random(shape) < dense).astype(np.int8)
+    kw = dict(niu=0.1, force=(1e-4, -2e-4, 1e-4), bc=bc, rho_bc=(1.002, 1.0, 1.001, 1.0, 1.0, 0.999),
+              vel_bc=((0, 0, 0), (0, 0, 0), (0, 0, 0), (1e-3, 0, 2e-3), (2e-3, 1e-3, 0), (0, 0, 0)), bc_form=bc_form,
+              visc_convention=1, guo_convention=2)
+    o = Oracle(oracle_params(shape, **kw), solid)
+    o.step(12)
+    lat = _native.Lattice(_native.make_params(shape, **kw))
+    lat.set_geometry(solid)
+    lat.init()
+    lat.step(12)
+    fl = solid == 0
+    for f, g in zip(("rho", "v"), lat.macros()):
+        assert np.array_equal(g[fl], o.field(f).astype(np.float32)[fl]), f
+    lat.close()
+
+
+@pytest.mark.parametrize("shape", [(512, 256, 1), (256, 64, 4)])
+def test_flat_lattices_need_few_records(shape):
+    """Only nodes of the x faces, and where a row starts anew, hold explicit links: 180 B of
+    populations and fields a node, 17 B of index and links, and no 80 B record each."""
+    lat = _native.Lattice(_native.make_params(shape, niu=0.1))
+    lat.set_geometry(np.zeros(shape, np.int8))
+    per_node = lat.info().device_bytes / np.prod(shape)
+    lat.close()
+    assert per_node < 205

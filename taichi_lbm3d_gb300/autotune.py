@@ -1,9 +1,11 @@
 """Autotuner for the batched step kernel.
 
 For each subvolume edge size it times the step kernel over a small
-batch of subvolumes of that size for every candidate (work-tile length, CTA
-size), with CUDA events on the batch's stream, and keeps the fastest.  Results
-are cached in a JSON file keyed by GPU name, storage mode and edge size
+batch of subvolumes of that size for every candidate (tile length, CTA
+size), with CUDA events on the batch's stream, and keeps the fastest.  A CTA
+steps one tile with a thread a node, so the candidates are the tiles up to the
+CTA size.  Results are cached in a JSON file keyed by GPU name, storage mode, edge
+size and kernel, so that timings of another kernel are not taken for this one's
 (default ``~/.cache/taichi_lbm3d_gb300/autotune.json``, or $LBM_AUTOTUNE_CACHE),
 so a later run with the same key does not time again.
 """
@@ -13,8 +15,13 @@ import time
 
 import numpy as np
 
-TILES = (256, 512, 1024, 2048, 4096)
-BLOCKS = (128, 256)
+TILES = (64, 128, 256)
+BLOCKS = (64, 128, 256)
+KERNEL = "tile-per-cta"     # changes with what the step kernel makes of (tile, block)
+
+
+def candidates():
+    return [(tile, block) for block in BLOCKS for tile in TILES if tile <= block]
 
 
 def cache_path():
@@ -52,6 +59,7 @@ def time_config(batch, tile, block, steps=20, warmup=4):
     batch.configure([tile] * batch.n, block)
     batch.init()
     batch.step(warmup, chunk=warmup)
+    batch.step(steps, chunk=steps)          # captures the graph that is timed
     stream = torch.cuda.ExternalStream(batch.stream())
     e0 = torch.cuda.Event(enable_timing=True)
     e1 = torch.cuda.Event(enable_timing=True)
@@ -71,19 +79,18 @@ def tune(solids_by_edge, storage="f16", force=(1e-6, 0, 0), niu=0.1, path=None, 
     gpu = _gpu_name()
     out = {}
     for edge, solids in sorted(solids_by_edge.items()):
-        key = "%s|%s|%d" % (gpu, storage, edge)
+        key = "%s|%s|%d|%s" % (gpu, storage, edge, KERNEL)
         if key in cache and not retune:
             out[edge] = cache[key]
             continue
         b = Batch(solids, niu=niu, force=force, storage=storage)
         best = None
         trials = {}
-        for block in BLOCKS:
-            for tile in TILES:
-                t = time_config(b, tile, block)
-                trials["%d/%d" % (tile, block)] = t * 1e3
-                if best is None or t < best[0]:
-                    best = (t, tile, block)
+        for tile, block in candidates():
+            t = time_config(b, tile, block)
+            trials["%d/%d" % (tile, block)] = t * 1e3
+            if best is None or t < best[0]:
+                best = (t, tile, block)
         nf = b.info()["n_fluid"]
         b.close()
         res = {"tile": best[1], "block": best[2], "ms_per_step": best[0] * 1e3,
@@ -98,12 +105,17 @@ def tune(solids_by_edge, storage="f16", force=(1e-6, 0, 0), niu=0.1, path=None, 
 
 
 def plan(edges, tuned):
-    """Per-subvolume tile lengths and one CTA size for a mixed batch: each
-    subvolume uses its edge's tile length; the CTA size is the one tuned for
-    the edge class holding the most cells."""
-    tiles = [int(tuned[e]["tile"]) for e in edges]
+    """Per-subvolume tile lengths and one CTA size for a mixed batch: the CTA size
+    is the one tuned for the edge class holding the most cells; each subvolume
+    uses its edge's tile length, the fastest at that CTA size where its trials
+    are at hand."""
     weight = {}
     for e in edges:
         weight[e] = weight.get(e, 0) + e ** 3
-    heavy = max(weight, key=weight.get)
-    return tiles, int(tuned[heavy]["block"])
+    block = int(tuned[max(weight, key=weight.get)]["block"])
+
+    def tile(t):
+        at = {int(k.split("/")[0]): ms for k, ms in t.get("trials_ms", {}).items() if int(k.split("/")[1]) == block}
+        return min(at, key=at.get) if at else int(t["tile"])
+
+    return [tile(tuned[e]) for e in edges], block

@@ -48,7 +48,7 @@ __device__ __forceinline__ int pull_source(const int32_t* __restrict__ map, cons
 #ifdef LBM_DEBUG
 // Debug builds (-DLBM_DEBUG): the first failed index check is recorded here
 // (1 = node coordinates outside the lattice, 2 = a map entry beyond the
-// fluid-node count) and read back by the host after the step; the offending
+// fluid-node count, 3 = a neighbour link beyond it) and read back by the host after the step; the offending
 // access is skipped.  One copy per translation unit; the single-phase step
 // (lbm_sp.cu) sets the node limit and reads the flag; elsewhere the limit
 // stays 0 and the check is off.

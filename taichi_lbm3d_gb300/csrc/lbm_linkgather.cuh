@@ -116,22 +116,34 @@ struct LinkGather {
         if constexpr (RAW) return Cd::template raw<S>(x);
         else return Cd::template dec<S>(x);
     }
+    // The source as decoded; debug builds take the node itself for one outside the
+    // nodes and record the failure (3).
+    static __device__ __forceinline__ int checked(int src, int n) {
+#ifdef LBM_DEBUG
+        if (g_lbm_debug_nlimit > 0 && (unsigned)src >= (unsigned)g_lbm_debug_nlimit) {
+            lbm_debug_fail(3);
+            return n;
+        }
+#endif
+        (void)n;
+        return src;
+    }
     template <int S>
     static __device__ __forceinline__ void one(R* F, const T* fin, int own, const NodeLinks& K, int n, const LinkRef<R>& rx) {
         const bool bounce = K.bits >> S & 1u;
-        const int a = bounce ? own + 32 * (lbm_lr(S) - S) : lbm_eoff32(K.template source<S>(n));
+        const int a = bounce ? own + 32 * (lbm_lr(S) - S) : lbm_eoff32(checked(K.template source<S>(n), n));
         F[S] = get<S>(fin[a + 32 * S]);
         if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), bounce ? rx.at : rx.template of<S>(), F[S]);
     }
     // Explicit sources of the links that the node word cannot express.
-    static __device__ __forceinline__ void recorded(R* F, const T* fin, const LbmLinks& L, const NodeLinks& K,
+    static __device__ __forceinline__ void recorded(R* F, const T* fin, const LbmLinks& L, const NodeLinks& K, int n,
                                                     const LinkRef<R>& rx) {
         if (!(K.bits & LBM_LINK_EXC)) return;
         const int4* rec = reinterpret_cast<const int4*>(K.record(L));
         int4 to;
 #define LBM_X(S, SRC)                                                                         \
     if (SRC >= 0) {                                                                           \
-        F[S] = get<S>(fin[lbm_eoff32(SRC) + 32 * S]);                                         \
+        F[S] = get<S>(fin[lbm_eoff32(checked(SRC, n)) + 32 * S]);                             \
         if constexpr (REF) F[S] = lbm_fma<R>((R)lbm_w(S), rx.template of<S>(), F[S]);         \
     }
         to = __ldg(rec);
@@ -154,7 +166,7 @@ struct LinkGather {
 #define LBM_G(S) one<S>(F, fin, own, K, n, rx);
         LBM_ALL_DIRS(LBM_G)
 #undef LBM_G
-        recorded(F, fin, L, K, rx);
+        recorded(F, fin, L, K, n, rx);
     }
 };
 

@@ -14,9 +14,9 @@
 // n + (n >> 5) * 576 + 32 s, lbm_common.cuh) in two buffers (ping-pong),
 // np = n_fluid padded to 64; neighbour links (lbm_links.cuh).  Per node and step
 // the kernel moves 19 loads + 19 stores of populations (152 B in FP32, 76 B in
-// 16-bit storage) and 9 B of links.  FP64, the staged kernels and LBM_DEBUG
-// builds find their sources through the dense int32 map cell -> node (or -1 for
-// solid) and packed node coordinates instead.
+// 16-bit storage) and 9 B of links.  FP64 and the staged kernels find their
+// sources through the dense int32 map cell -> node (or -1 for solid) and packed
+// node coordinates instead.
 //
 // Consecutive steps use programmatic dependent launch: a step's CTAs load their
 // links while the previous step drains, then wait for it.  Measured on the map
@@ -124,7 +124,7 @@ __device__ __forceinline__ void sp_finish_node(typename Codec<STORE>::R* F, int 
                                           lbm_ref_at(sp_ref(C), i), C, fout, vprev, rho_out, v_out);
 }
 
-// The step through the dense map: FP64, and every storage in LBM_DEBUG builds.
+// The step through the dense map: FP64.
 template <int STORE, int FORCE, bool MACROS>
 __global__ void __launch_bounds__(256)
     sp_step_kernel(const __grid_constant__ SpConsts<typename Codec<STORE>::R> C,
@@ -206,6 +206,12 @@ __global__ void __launch_bounds__(LINK_THREADS, FORCE && !Codec<STORE>::DEV ? LB
     K.load(L, n);
     int i = 0;
     if constexpr (REF) i = lbm_pi(__ldg(coord + n));
+#ifdef LBM_DEBUG
+    if (const uint32_t pc = __ldg(coord + n); lbm_pi(pc) >= C.nx || lbm_pj(pc) >= C.ny || lbm_pk(pc) >= C.nz) {
+        lbm_debug_fail(1);
+        return;
+    }
+#endif
     constexpr bool RAW = Cd::SCALE != 1;
     LinkRef<float> rx(sp_ref(C), i, C.nx);
     if constexpr (RAW) rx.scale((float)Cd::SCALE);
@@ -748,12 +754,7 @@ int run_steps(LbmHandle* h, int32_t n, bool macros_last) {
     if (rc0) return rc0;
 #endif
     if (h->tiled) return run_tiles<STORE>(h, n, macros_last);
-#ifdef LBM_DEBUG
-    constexpr bool LINKS = false;   // debug builds keep the kernel whose map lookups they check
-#else
-    constexpr bool LINKS = STORE != LBM_STORE_F64;   // the links gather into FP32
-#endif
-    if constexpr (LINKS) {
+    if constexpr (STORE != LBM_STORE_F64) {   // the links gather into FP32
         return run_links<STORE>(h, n, macros_last);
     } else {
         using R = typename Codec<STORE>::R;
@@ -918,8 +919,9 @@ int sp_debug_take(LbmHandle* h) {
     if (!rc && flag) {
         rc = lbm_cuda_check(h, cudaMemcpyToSymbol(g_lbm_debug, &zero, sizeof(int)), "debug flag");
         if (!rc)
-            rc = lbm_set_err(h, LBM_EINVAL, flag == 1 ? "debug check: node coordinates outside the lattice"
-                                                      : "debug check: neighbour map entry beyond the fluid-node count");
+            rc = lbm_set_err(h, LBM_EINVAL, flag == 1   ? "debug check: node coordinates outside the lattice"
+                                            : flag == 2 ? "debug check: neighbour map entry beyond the fluid-node count"
+                                                        : "debug check: neighbour link beyond the fluid-node count");
     }
     return rc;
 #else

@@ -116,7 +116,8 @@ __global__ void __launch_bounds__(GREY_THREADS, STORE == LBM_STORE_F64 ? 2 : 8) 
         j = lbm_pj(pc);
         k = lbm_pk(pc);
     }
-    const LinkRef<R> rx(sp_ref(C), i, C.nx);
+    LinkRef<R> rx;
+    if constexpr (Cd::RHOREF) rx = LinkRef<R>(sp_ref(C), i, C.nx, K);
     const int64_t np = C.np;
     const auto* fin = wait_previous(f_prev);
 

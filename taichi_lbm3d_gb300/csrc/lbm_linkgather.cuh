@@ -39,14 +39,14 @@ struct NodeLinks {
         w = x.x;
         bits = x.y;
         lane = n & (LBM_LINK_GROUP - 1);
-        // found without a vote, since which lanes are together at a vote is not
-        // fixed, and here, since looked up after the gather its latency adds to a
-        // step (24 x 192 x 192 all fluid, f32dev: 30.2 us, 27.7 here)
-        slot = 0;
-        if (bits & LBM_LINK_EXC) {
-            const int2 r = __ldg(reinterpret_cast<const int2*>(L.recs + n / LBM_LINK_GROUP));
-            slot = r.x + __popc((uint32_t)r.y & ((1u << lane) - 1u));
-        }
+        slot = bits & LBM_LINK_EXC ? find(L, n) : 0;
+    }
+    // Found without a vote, since which lanes are together at a vote is not fixed;
+    // with the links, since after the gather its latency adds to a step (24 x 192 x
+    // 192 all fluid, f32dev: 30.2 us, 27.7 so).
+    __device__ __forceinline__ int find(const LbmLinks& L, int n) const {
+        const int2 r = __ldg(reinterpret_cast<const int2*>(L.recs + n / LBM_LINK_GROUP));
+        return r.x + __popc((uint32_t)r.y & ((1u << lane) - 1u));
     }
     // Node across in row r.
     template <int RW>
@@ -70,7 +70,8 @@ struct NodeLinks {
             return rank<rw>();
         }
     }
-    __device__ __forceinline__ const int32_t* record(const LbmLinks& L) const {
+    __device__ __forceinline__ const int32_t* record(const LbmLinks& L) const { return record(L, slot); }
+    static __device__ __forceinline__ const int32_t* record(const LbmLinks& L, int slot) {
         return L.rec + (int64_t)LBM_LINK_REC * slot;
     }
     // Whether to take the code that looks for records: it serves every node, the
@@ -79,17 +80,20 @@ struct NodeLinks {
 };
 
 // Reference density of the 16-bit codecs at a node and its sources at x - 1 and
-// x + 1: stepped from the node's own value in a warp without an x face, from
+// x + 1: stepped from the node's own value in a group without an x face, from
 // the wrapped x in the others (the rounding of gather_node).
 template <typename R>
 struct LinkRef {
-    R at, xm, xp;
+    R at = (R)0, xm = (R)0, xp = (R)0;
     LinkRef() = default;
-    __device__ __forceinline__ LinkRef(const LbmRef<R>& ref, int i, int nx) {
-        const bool inside = __all_sync(__activemask(), i > 0 && i < nx - 1);
+    __device__ __forceinline__ LinkRef(const LbmRef<R>& ref, int i, int nx, const NodeLinks& K) {
         at = lbm_ref_at(ref, i);
-        xm = inside ? at - ref.b : lbm_fma<R>(ref.b, (R)(i == 0 ? nx - 1 : i - 1), ref.a);
-        xp = inside ? at + ref.b : lbm_fma<R>(ref.b, (R)(i == nx - 1 ? 0 : i + 1), ref.a);
+        xm = at - ref.b;
+        xp = at + ref.b;
+        if (K.w & LBM_LINK_XFACE) {
+            xm = lbm_fma<R>(ref.b, (R)(i == 0 ? nx - 1 : i - 1), ref.a);
+            xp = lbm_fma<R>(ref.b, (R)(i == nx - 1 ? 0 : i + 1), ref.a);
+        }
     }
     __device__ __forceinline__ void scale(R k) {
         at = at * k;
@@ -139,7 +143,9 @@ struct LinkGather {
     static __device__ __forceinline__ void recorded(R* F, const T* fin, const LbmLinks& L, const NodeLinks& K, int n,
                                                     const LinkRef<R>& rx) {
         if (!(K.bits & LBM_LINK_EXC)) return;
-        const int4* rec = reinterpret_cast<const int4*>(K.record(L));
+        // (with a reference density there is no register for the slot: 256^3 pack BF16
+        // 146.2 us, 8 bytes spilled, against 141.5)
+        const int4* rec = reinterpret_cast<const int4*>(K.record(L, REF ? K.find(L, n) : K.slot));
         int4 to;
 #define LBM_X(S, SRC)                                                                         \
     if (SRC >= 0) {                                                                           \

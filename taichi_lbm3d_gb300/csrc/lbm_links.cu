@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int 
         }
     }
     int start[8];
-    uint32_t w0 = 0, w1 = 0, far = 0;
+    uint32_t w0 = __any_sync(0xffffffffu, live && (i == 0 || i == B.nx - 1)) ? LBM_LINK_XFACE : 0u, w1 = 0, far = 0;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         int rank = -1;

@@ -29,11 +29,12 @@
 #define LBM_LINK_GROUP 32
 #define LBM_LINK_REC 20
 // LbmLinkNode.y: bit 0 as here, bits 1..18 the directions, 22..31 rows 6 and 7;
-// .x: rows 0..5 at 5 bits each.
+// .x: rows 0..5 at 5 bits each, bit 30 as here.
 #define LBM_LINK_EXC 1u              // the node has a record
 #define LBM_LINK_FACE (1u << 19)     // on a face with a boundary condition
 #define LBM_LINK_PRESSURE (1u << 20) // on a fixed-pressure face
 #define LBM_LINK_EDGE (1u << 21)     // on a face of the lattice
+#define LBM_LINK_XFACE (1u << 30)    // (.x) some node of the group is on an x face
 
 struct __align__(16) LbmLinkHead {
     int32_t start[8];  // rows ordered as lbm_link_ey / lbm_link_ez

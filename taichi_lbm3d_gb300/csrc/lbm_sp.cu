@@ -213,7 +213,8 @@ __global__ void __launch_bounds__(LINK_THREADS, FORCE && !Codec<STORE>::DEV ? LB
     }
 #endif
     constexpr bool RAW = Cd::SCALE != 1;
-    LinkRef<float> rx(sp_ref(C), i, C.nx);
+    LinkRef<float> rx;
+    if constexpr (REF) rx = LinkRef<float>(sp_ref(C), i, C.nx, K);
     if constexpr (RAW) rx.scale((float)Cd::SCALE);
     const auto* fin = wait_previous(f_prev);
     float F[19];

@@ -418,7 +418,8 @@ __global__ void __launch_bounds__(128, STORE == LBM_STORE_F64 ? 2 : LBM_TP_MINBL
         j = lbm_pj(pc);
         k = lbm_pk(pc);
     }
-    const LinkRef<R> rx(sp_ref(C), i, C.nx);
+    LinkRef<R> rx;
+    if constexpr (Cd::RHOREF) rx = LinkRef<R>(sp_ref(C), i, C.nx, K);
     const int64_t np = C.np;
     // rho_r, rho_b, psi of the colour launch; f, v of the previous step
     const auto* fin = wait_previous(f_prev);

@@ -1,6 +1,6 @@
 // Builds the neighbour links (lbm_links.cuh) of a lattice from its dense map
 // and packed coordinates: one warp per group of 32 nodes, two passes (tables
-// and record counts, then the records).
+// and record counts, then the records of the groups that have some).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -62,6 +62,8 @@ template <bool FILL>
 __global__ void __launch_bounds__(128) link_build_kernel(const LinkBuild B, int ngroup) {
     const int group = (blockIdx.x * 128 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (group >= ngroup) return;
+    if constexpr (FILL)
+        if (B.recs[group].lanes == 0) return;
     const int n = group * LBM_LINK_GROUP + lane;
     const bool live = n < B.n_fluid;
     const uint32_t pc = live ? B.coord[n] : 0u;

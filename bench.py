@@ -274,7 +274,7 @@ def batched(n_sub=256, seeds0=4000, fp64_subset=16, storage="f16", tol=1e-6, che
             max_steps=100_000, log=lambda m: print(m, file=sys.stderr, flush=True)):
     """Batched permeability: n_sub seeded subvolumes (edges {48..160}, r U[3,8], phi
     U[0.25,0.5]), fx = 1e-6, periodic, niu 0.1, each to steady state:
-    one persistent graph-captured batch (autotuned) against a serial loop of the
+    one graph-captured batch (autotuned) against a serial loop of the
     plain FP32 kernel; per-sample k error against FP64 on a subset."""
     from taichi_lbm3d_gb300 import autotune
     from taichi_lbm3d_gb300.batch import Batch, subvolume_solids
@@ -330,7 +330,7 @@ def batched(n_sub=256, seeds0=4000, fp64_subset=16, storage="f16", tol=1e-6, che
     total_updates = float(np.sum([int((s == 0).sum()) * n for s, n in zip(solids, st_b)]))
     return {"n_sub": n_sub, "edges": {str(e): edges.count(e) for e in sorted(set(edges))},
             "n_fluid_total": int(nf_all), "storage": storage, "block": block,
-            "tiles": {str(e): int(tuned[e]["tile"]) for e in sorted(tuned)},
+            "tiles": {str(e): t for e, t in sorted(zip(edges, tiles))},
             "batched_seconds": secs_b, "batched_mlups": total_updates / secs_b / 1e6,
             "batched_converged": int(cv_b.sum()), "serial_f32_seconds": secs_s,
             "wall_time_ratio_serial_over_batched": secs_s / secs_b,
@@ -735,7 +735,7 @@ def main():
     ap.add_argument("--convergence", action="store_true",
                     help="run the 256^3 pack to steady state in FP64/FP32/FP16/BF16 and print k errors")
     ap.add_argument("--batched", action="store_true",
-                    help="256 subvolumes to steady state: batched persistent launch vs serial plain kernel, k error vs FP64")
+                    help="256 subvolumes to steady state: batched launch vs serial plain kernel, k error vs FP64")
     ap.add_argument("--n-sub", type=int, default=256)
     ap.add_argument("--two-phase", action="store_true", help="131^3 two-phase drainage vs FP64")
     ap.add_argument("--grey", action="store_true", help="grey-scale (partial bounce-back) step on a 256^3 grey field")

@@ -205,7 +205,7 @@ int lbm_batch_create(const LbmParams* params, int32_t n_sub, const int32_t* dims
                      LbmBatch** out);
 int lbm_batch_destroy(LbmBatch* b);
 /* Tile length in nodes per subvolume (at most the CTA's threads) and CTA size of the kernel
- * (chosen by the autotuner in taichi_lbm3d_gb300/autotune.py). */
+ * (chosen by the autotuner in taichi_lbm3d_gb300/autotune.py), at any time between steps. */
 int lbm_batch_configure(LbmBatch* b, const int32_t* tile_len, int32_t block);
 /* Rest state f = feq(1, 0) in every subvolume, all subvolumes active. */
 int lbm_batch_init(LbmBatch* b);

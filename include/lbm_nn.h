@@ -61,7 +61,9 @@ int lbm_nn_pool2(const void* in, void* out, uint8_t* arg, int32_t n, int32_t d, 
 int lbm_nn_pool2_bwd(const void* gout, const uint8_t* arg, void* gin, const void* mask, int32_t n, int32_t d,
                      int32_t h, int32_t w, int32_t c, int32_t accumulate, void* stream);
 /* 2x nearest upsample (dims are the low-resolution ones) and its gradient,
- * multiplied by (mask > 0) when mask (low resolution) is given. */
+ * multiplied by (mask > 0) when mask (low resolution) is given.  (The package's
+ * network takes lbm_nn_upcat; these two, lbm_nn_concat, lbm_nn_split and lbm_nn_adam are
+ * for callers that need the parts, and what the tests compare the joined calls with.) */
 int lbm_nn_upsample2(const void* in, void* out, int32_t n, int32_t d, int32_t h, int32_t w, int32_t c, void* stream);
 int lbm_nn_upsample2_bwd(const void* gout, void* gin, const void* mask, int32_t n, int32_t d, int32_t h, int32_t w,
                          int32_t c, void* stream);

@@ -71,7 +71,7 @@ using namespace lbmk;
 // fluid nodes, body force), MLUPS, against a persistent grid whose CTAs claimed
 // 1024-node tiles from a counter and looked sources up in the dense maps: FP16
 // 42.0k / 32.0k, FP32 deviation form 37.9k / 30.9k, FP32 31.0k / 20.2k.  Bound by
-// issue slots as the single-lattice kernel.  Tiles of 64 and 128 threads run
+// issue (75% of the slots) and latency as the single-lattice kernel.  Tiles of 64 and 128 threads run
 // alike, of 256 5% slower.
 template <int STORE, int FORCE, bool CHECK>
 __global__ void __launch_bounds__(256, STORE == LBM_STORE_F64 ? 1 : FORCE && !Codec<STORE>::DEV ? 4 : 5)

@@ -17,11 +17,11 @@
 namespace {
 std::mutex g_err_mu;
 
-// L2 residency of the neighbour map.  The 18 map lookups of every node sit on
-// the step's critical path (coordinates -> map -> populations) and the map
-// (4 B per cell) is otherwise evicted by the populations streaming through L2
-// every step.  Each handle marks its map as a persisting access-policy window
-// on its stream; the process-wide set-aside (a limit of this process's CUDA
+// L2 residency of the neighbour map, for the steps that look it up (FP64 and the
+// staged kernels): the 18 lookups of every node sit on their critical path
+// (coordinates -> map -> populations) and the map (4 B per cell) is otherwise
+// evicted by the populations streaming through L2 every step.  Such a handle marks
+// its map as a persisting access-policy window on its stream; the process-wide set-aside (a limit of this process's CUDA
 // context, released when the process exits) is the largest map in use, capped
 // at the device maximum, and is returned to 0 when the last handle on the
 // device that used it is destroyed.  Best effort: failures only skip it.
@@ -295,8 +295,8 @@ int lbm_create(const LbmParams* params, LbmHandle** out) {
     h->elem = store_elem(params->storage);
     h->f64 = params->storage == LBM_STORE_F64;
     h->force = params->force[0] != 0 || params->force[1] != 0 || params->force[2] != 0;
-    /* 128-thread CTAs measured 1.9% faster than 256 on the single-phase step
-       (same 1536 resident threads per SM); the two-phase kernels keep 256. */
+    /* 128-thread CTAs measured 1.9% faster than 256 on the map step (same 1536
+       resident threads per SM); the link kernels take at most 128 whatever is asked. */
     h->block = params->block_size ? params->block_size : (params->two_phase ? 256 : 128);
     h->ncell = (int64_t)params->nx * params->ny * params->nz;
     cudaSetDevice(h->device);

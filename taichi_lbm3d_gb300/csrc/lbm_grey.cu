@@ -86,7 +86,8 @@ __device__ __forceinline__ void grey_face_restore(R* F, int i, int j, int k, con
 // 28.7k FP32 deviation form at 7).  192^3 grey field, MLUPS against the map
 // kernel with IEEE divisions and the dense Guo term: FP32 forced along x 25.1k /
 // 18.3k, FP32 with pressure faces 26.4k / 23.5k, FP32 deviation form 30.3k / 26.9k,
-// FP16 29.9k / 25.7k.  Bound by issue slots and latency: 55 loads a node.
+// FP16 29.9k / 25.7k.  Bound by issue (74% of the slots, 1118 instructions a node) and
+// the latency of 55 loads a node.
 constexpr int GREY_THREADS = 128;
 
 template <int STORE, int FORCE, bool MACROS>

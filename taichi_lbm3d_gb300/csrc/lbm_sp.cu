@@ -167,22 +167,24 @@ __global__ void __launch_bounds__(256, 1)
 // ------------------------------------------------------------ link step
 // The step of all storages but FP64: the pull sources come from the neighbour
 // links (lbm_links.cuh, 9 bytes a node read in order) instead of coordinates and
-// 18 map lookups.  What that buys is instructions (877 against 1052 per warp of
-// 32 nodes, FP32; 717 against 890, FP32 deviation form) and one dependent load
-// less before the populations.  256^3 pack, MLUPS, map kernel / links / links with one
+// 18 map lookups.  What that buys is instructions (731 a node against 962, FP32;
+// 568 in the FP32 deviation form) and one dependent load less before the
+// populations.  256^3 pack, MLUPS, map kernel / links / links with one
 // reciprocal per density instead of three to six IEEE divisions: FP32 33.6k /
-// 35.5k / 36.9k, FP32 deviation form 35.1k / 36.1k / 38.7k, FP16 32.2k / 39.9k /
-// 40.6k; 64^3 cavity FP32 30.1k / 34.3k / 33.7k (launch-bound); channel 101 x 67 x 53,
-// FP32 forced along x 19.3k / 21.3k / 28.7k (with the x-only Guo term).
-// FP32 then moves 167 B a node at 0.92 of the copy bandwidth (DRAM-bound); the
-// 16-bit storages are bound by issue slots (87% of them used).  Two nodes per
+// 35.5k / 37.3k, FP32 deviation form 35.1k / 36.1k / 39.2k, FP16 32.2k / 39.9k /
+// 41.3k; 64^3 cavity FP32 30.1k / 34.3k / 34.6k (launch-bound); channel 101 x 67 x 53,
+// FP32 forced along x 19.1k / 21.3k / 29.4k (with the x-only Guo term).
+// FP32 then moves 165 B a node at 0.91 of the copy bandwidth (DRAM-bound); the
+// 16-bit storages move 94 B and issue in 77% of the slots, with 3.5 warps waiting
+// for loads per issue: issue and latency together.  Two nodes per
 // thread in packed FP32 halve the instructions and were slower (28.0k FP32, 96
 // registers: half the warps, each living longer), pushing instead of pulling
 // too (19.5k: unaligned stores leave partly written sectors).
 //
 // Resident 128-thread CTAs per SM, measured on the same lattices: 10 (48
-// registers, no spill; FP32 36.9k against 36.0k at 9 and 36.2k at 11, FP16 40.6k
-// against 40.3k and 37.4k), forced FP32 reference arithmetic 9 (28.7k; 28.2k at 10).
+// registers, no spill; FP32 37.3k against 36.1k at 9 and 36.6k at 11, FP16 41.3k
+// against 40.2k and 39.5k), forced FP32 reference arithmetic 9 (29.4k; 29.4k at 8,
+// 28.9k at 10).
 #ifndef LBM_LINK_MINBLOCKS
 #define LBM_LINK_MINBLOCKS 10
 #endif
@@ -865,7 +867,7 @@ int sp_launch_init(LbmHandle* h, const void* rho_nodes, const void* v_nodes) {
 
 // Per-tile staging plan of the staged step kernels (after the index is built),
 // chosen by LBM_SP_TILED in the environment: 0 or unset = sp_link_kernel (the
-// default: 36.9k / 38.7k / 40.6k), 1 = persistent staged kernel, 2 = one staged tile
+// default: 37.3k / 39.2k / 41.3k), 1 = persistent staged kernel, 2 = one staged tile
 // per CTA.  256^3 pack, FP32 / f32dev / FP16 MLUPS on one GB300: sp_step_kernel
 // 34.6k / 35.4k / 31.8k; persistent staged 29.2k / 29.9k / 29.4k; one tile per
 // CTA 28.6k / 28.9k / 28.4k, and 32.3k / 32.9k / 29.1k when that kernel stages

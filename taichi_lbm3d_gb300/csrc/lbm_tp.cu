@@ -28,11 +28,11 @@
 // only when the caller reads them next (MACROS) or, for v, where a pressure
 // face needs the previous step's.
 //
-// 131^3 drainage, FP32, 894k nodes: 81.8 us a step against 98.4 with six scalar
+// 131^3 drainage, FP32, 898k nodes: 81.0 us a step against 98.4 with six scalar
 // loads a direction and map lookups.  Launch A is bound by L1 wavefronts (every
-// direction reads its own 24 unaligned bytes: 68% of the data pipe), launch B by
-// issue slots and latency; its psi loads wait together with the
-// populations' (after the faces 83.0 us).  Storing the 38 recoloured
+// direction reads its own 24 unaligned bytes: 71% of the data pipe, 65% of the
+// issue slots), launch B by issue slots (66%) and latency at 72 registers; its psi
+// loads wait together with the populations' (after the faces 83.0 us).  Storing the 38 recoloured
 // populations instead (two values a direction in launch A) took a third of the
 // wavefronts but 140 MB more DRAM traffic a step: 94 us.
 #include <cuda_runtime.h>
@@ -43,7 +43,8 @@
 #include "lbm_linkgather.cuh"
 
 // Resident 128-thread CTAs per SM of the two launches (FP32 and 16-bit), us a step
-// on the same lattice / on a 50 x 44 x 37 sample: 10 and 7 81.8 / 13.3; 10 and 8
+// on the same lattice / on a 50 x 44 x 37 sample, before records were looked up with
+// the links (81.0 / 13.1 since): 10 and 7 81.8 / 13.3; 10 and 8
 // 81.7 / 14.6; 10 and 9 86.6 / 16.4; 10 and 6 87.5 / 15.6; 9 and 7 88.1, 12 and 7 84.2.
 #ifndef LBM_TP_MINBLOCKS_A
 #define LBM_TP_MINBLOCKS_A 10

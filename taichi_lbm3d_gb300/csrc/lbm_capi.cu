@@ -238,7 +238,9 @@ int step_graph_launch(LbmHandle* h) {
             return 1;
         }
         const int cur = h->cur;
+        h->step_capture = true;
         const int rc = launch_steps(h, STEP_GRAPH, false);
+        h->step_capture = false;
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamEndCapture(h->stream, &g);
         h->cur = cur;

@@ -85,6 +85,7 @@ struct LbmHandle {
     void* d_f[2] = {nullptr, nullptr};     // populations, 19 x np elements in AoSoA-32 chunks
     int cur = 0;
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};   // a run of steps from each buffer order (lbm_capi.cu)
+    bool step_capture = false;             // such a run is being captured
     void* d_vprev = nullptr;               // [3][np] previous-step v (pressure faces)
     void* d_rho = nullptr;                 // [np]
     void* d_v = nullptr;                   // [3][np]

@@ -618,7 +618,13 @@ int launch_step(LbmHandle* h, const SpConsts<typename Codec<STORE>::R>& C, int g
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = LBM_SP_PDL ? 1 : 0;
+    // In a replayed run launches follow at once, and CTAs that become resident while a
+    // step of at most one a SM still runs land beside its own: FP64 is bound by each
+    // SM's FP64 units, so two on one take twice as long (24^3 79.5 us a step, 35.5 one
+    // after the other; 20^3 41.6 and 35.6).  Single launches gain more from the overlap
+    // (16^3 unforced 19.5 against 22.6).
+    const bool overlap = !(h->step_capture && grid <= h->sm_count);
+    cfg.numAttrs = LBM_SP_PDL && overlap ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, sp_step_kernel<STORE, FORCE, MACROS>, C, fin, fout,
                                              (const int32_t*)h->d_map, (const uint32_t*)h->d_coord, (R*)h->d_vprev,
                                              (R*)h->d_rho, (R*)h->d_v);

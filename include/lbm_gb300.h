@@ -210,7 +210,7 @@ int lbm_batch_configure(LbmBatch* b, const int32_t* tile_len, int32_t block);
 /* Rest state f = feq(1, 0) in every subvolume, all subvolumes active. */
 int lbm_batch_init(LbmBatch* b);
 /* nsteps steps of the active subvolumes, in graph launches of `chunk` steps
- * (use_graph = 1) or plain launches (0). */
+ * (use_graph = 1) or plain launches (0); LBM_ESTATE before lbm_batch_init. */
 int lbm_batch_step(LbmBatch* b, int32_t nsteps, int32_t chunk, int32_t use_graph);
 /* Run until each subvolume's FP64 Darcy velocity along x changes by <= tol
  * between checks; converged subvolumes drop out of the work list.  Per
